@@ -843,9 +843,10 @@ int gabe_meansvars(gabe_handle *h, double out4[4]) {
     if (!h->uploaded) return set_err(h, GABE_ERR_STATE, "meansvars before upload");
     CK(h, cudaSetDevice(h->dev));
     const OutArgs a = out_args(h);
-    const int nblocks = 148 * 8;  // partials hold >= 2 * nblocks doubles
-    for (int pass = 0; pass < 2; pass++)
-        CK(h, h->f32 ? meansvars_f32(a, pass, nblocks, h->stream) : meansvars_f64(a, pass, nblocks, h->stream));
+    const int nblocks = 148 * 8;  // partials hold >= 4 * nblocks doubles
+    if (h->f32) CK(h, meansvars_f32(a, nblocks, h->stream));
+    else
+        for (int pass = 0; pass < 2; pass++) CK(h, meansvars_f64(a, pass, nblocks, h->stream));
     double r[4];
     CK(h, cudaMemcpyAsync(r, h->outres, sizeof(r), cudaMemcpyDeviceToHost, h->stream));
     CK(h, cudaStreamSynchronize(h->stream));
@@ -915,7 +916,7 @@ int gabe_spectra_raw(gabe_handle *h, double *sums, double *counts, int nbins, in
     b.zero_re[0] = h->lc.gridsize * s.fbar[0];
     b.zero_re[1] = h->lc.gridsize * s.fbar[1];
     const size_t smem = (size_t)h->nbins * (ns * 8 + 4);
-    Launch lb{dim3(kBinBlocks), dim3(256), smem, h->stream};
+    Launch lb{dim3(kBinBlocks), dim3(kBinThreads), smem, h->stream};
     CK(h, h->f32 ? bins_f32(b, lb) : bins_f64(b, lb));
     double *dsum = h->bin_sum, *dcnt = h->bin_sum + 3 * h->nbins;
     CK(h, bin_reduce(h->bin_part, h->bin_cnt_part, kBinBlocks, ns, h->nbins, dsum, dcnt, h->stream));

@@ -23,6 +23,7 @@
 #include <math_constants.h>
 
 #include "kspace.cuh"
+#include "spectra.cuh"
 #include "sweep32.cuh"
 
 namespace gabe {
@@ -295,32 +296,11 @@ __global__ void __launch_bounds__(256) ens_bin_kernel(EnsBinArgs a) {
     for (int q = threadIdx.x; q < nb; q += blockDim.x) hc[q] = 0u;
     __syncthreads();
     const EnsLat &E = a.lat[blockIdx.y];
-    const int N = E.N, nz = N / 2 + 1;
-    const size_t M = (size_t)N * N * nz;
+    const int N = E.N;
     const Cplx<float> *F = reinterpret_cast<const Cplx<float> *>(E.S);
     const double zre[2] = {E.c.gridsize * E.sc->fbar[0], E.c.gridsize * E.sc->fbar[1]};
-    for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < M; idx += (size_t)a.nblk * blockDim.x) {
-        const int kz = (int)(idx % nz);
-        const size_t t = idx / nz;
-        const int j = (int)(t % N), i = (int)(t / N);
-        const int px = i <= N / 2 ? i : i - N, py = j <= N / 2 ? j : j - N;
-        const int b = (int)sqrt((double)px * px + (double)py * py + (double)kz * kz);
-        const bool edge = (kz == 0) || (kz == N / 2);
-        const double w = edge ? 1.0 : 2.0;
-        atomicAdd(&hc[b], edge ? 1u : 2u);
-        for (int f = 0; f < 2; f++) {
-            double re = (double)F[(size_t)f * M + idx].re, im = (double)F[(size_t)f * M + idx].im;
-            if (idx == 0) re += zre[f];
-            atomicAdd(&hs[f * nb + b], w * (re * re + im * im));
-        }
-        if (E.G) {
-            const size_t src = (a.quirk && kz == 0) ? idx + (size_t)(N / 2) : idx;
-            const Cplx<float> lp = E.G[2 * M + src], lx = E.G[3 * M + src];
-            const double p =
-                2. * (((double)lp.re * lp.re + (double)lp.im * lp.im) + ((double)lx.re * lx.re + (double)lx.im * lx.im));
-            atomicAdd(&hs[2 * nb + b], w * p);
-        }
-    }
+    bin_points<float>(F, E.G, N, N, 0, 0, a.quirk, zre, nb, hs, hc, blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32,
+                      a.nblk * (blockDim.x / 32));
     __syncthreads();
     double *ps = a.part + ((size_t)blockIdx.y * a.nblk + blockIdx.x) * 3 * nb;
     unsigned int *pc = a.part_cnt + ((size_t)blockIdx.y * a.nblk + blockIdx.x) * nb;

@@ -118,8 +118,8 @@ cudaError_t from_fluct(const float *x, size_t n, const double *mean, double *out
     return cudaGetLastError();
 }
 
-cudaError_t meansvars_f32(const OutArgs &a, int pass, int nblocks, cudaStream_t s) {
-    meansvars_kernel<float><<<nblocks, 256, 0, s>>>(a, pass);
+cudaError_t meansvars_f32(const OutArgs &a, int nblocks, cudaStream_t s) {
+    meansvars_fluct_kernel<<<nblocks, 256, 0, s>>>(a);
     return cudaGetLastError();
 }
 

@@ -83,12 +83,12 @@ cudaError_t configure_bins(size_t max_smem) {
 cudaError_t bin_reduce(const double *part_sum, const unsigned int *part_cnt, int nblocks, int nseries, int nbins,
                        double *sum, double *cnt, cudaStream_t s) {
     const int n = nseries * nbins;
-    bin_reduce_kernel<<<(n + 127) / 128, 128, 0, s>>>(part_sum, part_cnt, nblocks, nseries, nbins, sum, cnt);
+    bin_reduce_kernel<<<(n + 31) / 32, 32 * kBinWays, 0, s>>>(part_sum, part_cnt, nblocks, nseries, nbins, sum, cnt);
     return cudaGetLastError();
 }
 
 cudaError_t meansvars_f64(const OutArgs &a, int pass, int nblocks, cudaStream_t s) {
-    meansvars_kernel<double><<<nblocks, 256, 0, s>>>(a, pass);
+    meansvars_kernel<<<nblocks, 256, 0, s>>>(a, pass);
     return cudaGetLastError();
 }
 

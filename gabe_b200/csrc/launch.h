@@ -175,7 +175,7 @@ cudaError_t gw_unpack_f32(const void *G, size_t cnt, size_t m0, int N, size_t M,
 
 // meansvars() and outputfield() rows on the device (output.cuh)
 cudaError_t meansvars_f64(const OutArgs &a, int pass, int nblocks, cudaStream_t s);
-cudaError_t meansvars_f32(const OutArgs &a, int pass, int nblocks, cudaStream_t s);
+cudaError_t meansvars_f32(const OutArgs &a, int nblocks, cudaStream_t s);
 cudaError_t slice_f64(const OutArgs &a, int nj, int nk, int skip, size_t r0, size_t cnt, double *out, cudaStream_t s);
 cudaError_t slice_f32(const OutArgs &a, int nj, int nk, int skip, size_t r0, size_t cnt, double *out, cudaStream_t s);
 

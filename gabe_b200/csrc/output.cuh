@@ -8,7 +8,7 @@
 // instantiations are compiled without FMA contraction).  FP32 storage holds
 // fluctuations d about the homogeneous values fbar: a field value is
 // fbar + d, its gradient that of d (the constant cancels), and its variance
-// sum (f^2 - av^2) = sum (d - dbar)(2 fbar + d + dbar) without cancellation.
+// that of d.
 #pragma once
 
 #include "common.cuh"
@@ -19,9 +19,9 @@ struct OutArgs {
     const void *X, *D;  // fields and momenta of the current stage 0, [2][N^3]
     const DevScalars *sc;
     LatticeConsts c;
-    double *partials;  // >= gridDim.x * 2 doubles
+    double *partials;  // >= gridDim.x * 4 doubles
     unsigned int *counter;
-    double *res;  // [8]: av[2], var[2], FP32: mean fluctuation[2]
+    double *res;  // [8]: av[2], var[2]
 };
 
 template <typename T>
@@ -31,32 +31,37 @@ __device__ __forceinline__ double field_value(const OutArgs &a, int fld, size_t 
     else return a.sc->fbar[fld] + (double)X[(size_t)fld * a.c.N * a.c.N * a.c.N + x];
 }
 
-// pass 0: av = sum f / N^3; pass 1: var = sum (f f - av av) / N^3, per field
-template <typename T>
-__global__ void __launch_bounds__(256) meansvars_kernel(OutArgs a, int pass) {
+// FP64 storage: pass 0: av = sum f / N^3; pass 1: var = sum (f f - av av) /
+// N^3, per field, the reference's two passes (the second needs the first's
+// mean, and its sum is dominated by that mean's rounding, so each thread's
+// order of additions is part of the result).  The loads of kMvUnroll
+// iterations are issued together, the additions stay in order.
+constexpr int kMvUnroll = 8;
+static __global__ void __launch_bounds__(256) meansvars_kernel(OutArgs a, int pass) {
     __shared__ double sred[8 * 2];
     __shared__ int sflag;
     const size_t n3 = (size_t)a.c.N * a.c.N * a.c.N;
-    const T *X = static_cast<const T *>(a.X);
+    const double *X = static_cast<const double *>(a.X);
     double acc[2] = {0., 0.};
 #pragma unroll
     for (int f = 0; f < 2; f++) {
-        const T *x = X + f * n3;
-        double av = 0., fb = 0., db = 0.;
-        if (pass == 1) {
-            av = a.res[f];
-            if constexpr (sizeof(T) == 4) {
-                fb = a.sc->fbar[f];
-                db = a.res[4 + f];
-            }
-        }
+        const double *x = X + f * n3;
+        const double av = pass == 1 ? a.res[f] : 0.;
+        const size_t stride = (size_t)gridDim.x * blockDim.x;
+        size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
         double s = 0.;
-        for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n3; q += (size_t)gridDim.x * blockDim.x) {
-            const double v = (double)x[q];
+        auto add = [&](double v) {
             if (pass == 0) s += v;
-            else if constexpr (sizeof(T) == 8) s += v * v - av * av;  // g2output.cpp:98
-            else s += (v - db) * (2. * fb + v + db);
+            else s += v * v - av * av;  // g2output.cpp:98
+        };
+        for (; q + (kMvUnroll - 1) * stride < n3; q += kMvUnroll * stride) {
+            double v[kMvUnroll];
+#pragma unroll
+            for (int u = 0; u < kMvUnroll; u++) v[u] = __ldg(x + q + u * stride);
+#pragma unroll
+            for (int u = 0; u < kMvUnroll; u++) add(v[u]);
         }
+        for (; q < n3; q += stride) add(x[q]);
         acc[f] = s;
     }
     block_reduce<2>(acc, sred);
@@ -68,18 +73,50 @@ __global__ void __launch_bounds__(256) meansvars_kernel(OutArgs a, int pass) {
     double tot[2];
     sum_partials<2>(a.partials, gridDim.x, tot, sred);
     if (threadIdx.x == 0) {
-        const double gs = a.c.gridsize;
+        for (int f = 0; f < 2; f++) a.res[pass == 0 ? f : 2 + f] = tot[f] / a.c.gridsize;  // g2output.cpp:92, :99
+        *a.counter = 0u;
+    }
+}
+
+// FP32 storage: with f = fbar + d both moments come from one read of the
+// fluctuations, av = fbar + <d> and sum (f^2 - av^2) / N^3 = <d^2> - <d>^2,
+// 16-byte loads (N^3 is a multiple of 16).  512^3: 0.157 ms (6.8 TB/s)
+// against 0.87 for two passes of 4-byte loads.
+static __global__ void __launch_bounds__(256) meansvars_fluct_kernel(OutArgs a) {
+    __shared__ double sred[8 * 4];
+    __shared__ int sflag;
+    const size_t n3 = (size_t)a.c.N * a.c.N * a.c.N, n4 = n3 / 4, stride = (size_t)gridDim.x * blockDim.x;
+    const float4 *X = static_cast<const float4 *>(a.X);
+    double acc[4] = {0., 0., 0., 0.};  // sum d per field, sum d^2 per field
+    auto add = [&](int f, const float4 v) {
+        const double d0 = v.x, d1 = v.y, d2 = v.z, d3 = v.w;
+        acc[f] += (d0 + d1) + (d2 + d3);
+        acc[2 + f] += (d0 * d0 + d1 * d1) + (d2 * d2 + d3 * d3);
+    };
+    size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    for (; q + stride < n4; q += 2 * stride) {
+        const float4 u0 = __ldg(X + q), u1 = __ldg(X + n4 + q), w0 = __ldg(X + q + stride),
+                     w1 = __ldg(X + n4 + q + stride);
+        add(0, u0);
+        add(1, u1);
+        add(0, w0);
+        add(1, w1);
+    }
+    for (; q < n4; q += stride) {
+        add(0, X[q]);
+        add(1, X[n4 + q]);
+    }
+    block_reduce<4>(acc, sred);
+    if (threadIdx.x == 0)
+        for (int v = 0; v < 4; v++) a.partials[4 * blockIdx.x + v] = acc[v];
+    if (!last_block_done(a.counter, &sflag)) return;
+    double tot[4];
+    sum_partials<4>(a.partials, gridDim.x, tot, sred);
+    if (threadIdx.x == 0) {
         for (int f = 0; f < 2; f++) {
-            if (pass == 0) {
-                if constexpr (sizeof(T) == 8) {
-                    a.res[f] = tot[f] / gs;  // g2output.cpp:92
-                } else {
-                    a.res[4 + f] = tot[f] / gs;
-                    a.res[f] = a.sc->fbar[f] + tot[f] / gs;
-                }
-            } else {
-                a.res[2 + f] = tot[f] / gs;  // g2output.cpp:99
-            }
+            const double db = tot[f] / a.c.gridsize;
+            a.res[f] = a.sc->fbar[f] + db;
+            a.res[2 + f] = tot[2 + f] / a.c.gridsize - db * db;
         }
         *a.counter = 0u;
     }

@@ -571,7 +571,7 @@ int gabe_slab_spectra_raw(gabe_slab *s, double *sums, double *counts) {
     b.zero_re[1] = s->lc.gridsize * d.fbar[1];
     b.m = s->nloc;
     b.y0 = s->plane0;
-    Launch lb{dim3(kSlabBinBlocks), dim3(256), (size_t)nb * (ns * 8 + 4), s->stream};
+    Launch lb{dim3(kSlabBinBlocks), dim3(kBinThreads), (size_t)nb * (ns * 8 + 4), s->stream};
     SCK(s, s->f32 ? bins_f32(b, lb) : bins_f64(b, lb));
     SCK(s, bin_reduce(s->bin_part, s->bin_cnt_part, kSlabBinBlocks, ns, nb, s->bin_sum, s->bin_sum + ns * nb, s->stream));
     SCK(s, cudaMemcpyAsync(sums, s->bin_sum, (size_t)ns * nb * 8, cudaMemcpyDeviceToHost, s->stream));

@@ -28,6 +28,7 @@ UNITS = [
     ("kernels_f32.cu", []),
     ("fft3d.cu", []),
     ("fftt.cu", []),
+    ("fftp.cu", []),
     ("noalloc.cu", ["-fmad=false"]),
     ("ensemble.cu", []),
     ("slab.cu", []),

@@ -60,6 +60,8 @@ struct gabe_handle {
     bool own_fft = false;   // the library's three-pass 3-D r2c (fft3d.cuh)
     bool fftt = false;      // the transposed three-pass transform with the pass along i fused into the
                             // k-space update (fftt.cuh); G is then kept as [4][kz][ky][kx]
+    bool fftp = false;      // the plane transform, lines along i fused into the k-space update (fftp.cuh)
+    int gt = 0;             // order of G (g_index): 1 with fftt, 2 with fftp
     void *fft_work = nullptr;
     size_t fft_work_bytes = 0;
     LatticeConsts lc{};
@@ -126,9 +128,9 @@ int make_plans(gabe_handle *h) {
     size_t ws_src = 0, ws_spec = 0;
     const cufftType t = h->f32 ? CUFFT_R2C : CUFFT_D2Z;
     // the library's in-layout three-pass r2c: on request
-    h->own_fft = h->evolve_gw && h->f32 && !h->fftt && fft3d_supported(h->N) && (h->p.flags & GABE_FLAG_OWN_FFT);
-    if (h->own_fft || h->fftt) {
-        // no plan: fft3d.cuh / fftt.cuh
+    h->own_fft = h->evolve_gw && h->f32 && !h->fftt && !h->fftp && fft3d_supported(h->N) && (h->p.flags & GABE_FLAG_OWN_FFT);
+    if (h->own_fft || h->fftt || h->fftp) {
+        // no plan: fft3d.cuh / fftt.cuh / fftp.cuh
     } else if (h->evolve_gw) {
         long long inem[3] = {N, N, 2 * nz}, onem[3] = {N, N, nz};
         CF(h, cufftCreate(&h->plan_src));
@@ -165,7 +167,7 @@ int fft_r2c(gabe_handle *h, cufftHandle plan, void *in, void *out) {
 // The GW chain of step n overlaps the field sweeps of step n+1 (two source
 // buffers) -- except with the library's FFT, which runs in line (measured
 // faster at 512^3) and uses the second buffer as its column passes' target.
-bool overlapped(const gabe_handle *h) { return h->evolve_gw && h->S2 != nullptr && !h->own_fft && !h->fftt; }
+bool overlapped(const gabe_handle *h) { return h->evolve_gw && h->S2 && !h->own_fft && !h->fftt && !h->fftp; }
 float *fft_scratch(const gabe_handle *h) { return h->own_fft ? static_cast<float *>(h->S2) : nullptr; }
 void *source_buffer(const gabe_handle *h, int slot) { return slot && h->S2 ? h->S2 : h->S; }
 
@@ -178,6 +180,14 @@ int source_fft(gabe_handle *h, int slot, cudaStream_t s) {
     if (h->fftt) {  // rows S -> S2, pass along j S2 -> S; the pass along i runs inside the k-space update
         CK(h, fftt_rows_f32(h->N, static_cast<const float *>(S), h->S2, 2 * kSrc, &h->sc->status, s));
         CK(h, fftt_cols_f32(h->N, h->S2, S, 2 * kSrc, &h->sc->status, s));
+        return GABE_OK;
+    }
+    if (h->fftp) {  // the planes of the stage-0 and of the stage-1 sources, S -> S2; the lines run in the k-space update
+        const int n = kSrc * h->N;
+        const size_t half = (size_t)kSrc * h->N * h->N * (h->N + 2);  // floats of one stage
+        for (int st = 0; st < 2; st++)
+            CK(h, fftp_planes_f32(h->N, static_cast<const float *>(S) + st * half, static_cast<float *>(h->S2) + st * half,
+                                  n, s));
         return GABE_OK;
     }
     if (h->own_fft) {
@@ -196,6 +206,10 @@ int kspace(gabe_handle *h, int slot, cudaStream_t s) {
     k.sc = h->sc;
     k.c = h->lc;
     k.slot = slot;
+    if (h->fftp) {
+        CK(h, fftp_lines_f32(h->N, h->S2, h->G, h->sc, nullptr, 1, h->lc, slot, s));
+        return GABE_OK;
+    }
     if (h->fftt) {
         CK(h, fftt_ikspace_f32(h->N, k.S, h->G, h->sc, h->lc, slot, &h->sc->status, s));
         return GABE_OK;
@@ -358,7 +372,7 @@ int upload_gw(gabe_handle *h, const double *h0, const double *l0) {
             for (int q = 0; q < 12; q++)
                 CK(h, cudaMemcpyAsync(stage + (size_t)q * cnt, src[w] + (size_t)q * M + m0, cnt * 8,
                                       cudaMemcpyHostToDevice, h->stream));
-            CK(h, h->f32 ? gw_pack_f32(stage, cnt, m0, h->N, M, h->G, w, h->gwnorm + 2 * w, h->fftt, h->stream)
+            CK(h, h->f32 ? gw_pack_f32(stage, cnt, m0, h->N, M, h->G, w, h->gwnorm + 2 * w, h->gt, h->stream)
                          : gw_pack_f64(stage, cnt, m0, h->N, M, h->G, w, h->gwnorm + 2 * w, h->stream));
         }
     }
@@ -382,7 +396,7 @@ int download_gw(gabe_handle *h, double *h0, double *l0) {
         if (!dst[w]) continue;
         for (size_t m0 = 0; m0 < M; m0 += chunk) {
             const size_t cnt = (M - m0) < chunk ? (M - m0) : chunk;
-            CK(h, h->f32 ? gw_unpack_f32(h->G, cnt, m0, h->N, M, w, stage, h->fftt, h->stream)
+            CK(h, h->f32 ? gw_unpack_f32(h->G, cnt, m0, h->N, M, w, stage, h->gt, h->stream)
                          : gw_unpack_f64(h->G, cnt, m0, h->N, M, w, stage, h->stream));
             for (int q = 0; q < 12; q++)
                 CK(h, cudaMemcpyAsync(dst[w] + (size_t)q * M + m0, stage + (size_t)q * cnt, cnt * 8,
@@ -501,17 +515,29 @@ int gabe_create(const gabe_params *p, gabe_handle **out) {
     }
     // sources need 10 padded slots; spectra need 2; uploads stage one FP64 field array
     h->evolve_gw = p->gws_on && p->expansion == 1;
-    // the transposed form: on request, and by default for FP32 at N >= 128 (measured fastest there:
-    // per step 8.1 against ~11 ms at 512^3, 1.21 against 1.41 at 256^3, 0.170 against 0.192 at 128^3
-    // with cuFFT's plan and the overlapped k-space chain; a tie at 64^3)
+    // the transposed form: on request, and by default for FP32 at N >= 256 (measured fastest there:
+    // per step 8.1 against ~11 ms at 512^3, 1.21 against 1.41 at 256^3 with cuFFT's plan and the
+    // overlapped k-space chain; 0.170 against 0.192 at 128^3, where the plane form is ahead of both;
+    // a tie with cuFFT's plan at 64^3)
     h->fftt = h->evolve_gw && h->f32 && fftt_supported(h->N) &&
               ((p->flags & GABE_FLAG_TRANSPOSED_FFT) ||
                (h->N >= 128 && !(p->flags & (GABE_FLAG_OWN_FFT | GABE_FLAG_CUFFT_3D))));
+    // the plane transform at the sizes it takes except 64 (transform and k-space update at 96^3 61 us against
+    // 108 with cuFFT's plan, at 128^3 114 against 120 with the transposed form), unless a flag names a form
+    h->fftp = h->evolve_gw && h->f32 && fftp_supported(h->N) && h->N != 64 &&
+              !(p->flags & (GABE_FLAG_OWN_FFT | GABE_FLAG_CUFFT_3D | GABE_FLAG_TRANSPOSED_FFT));
+    if (h->fftp) h->fftt = false;
     h->nslots = h->evolve_gw ? 2 * kSrc : 2;
     h->S_bytes = (size_t)h->nslots * p->N * p->N * (p->N + 2) * h->esz;
     if ((rc = dalloc(h, &h->S, h->S_bytes))) return bail(rc);
     if (h->fftt) {  // the transposed transform's first pass writes out of place
         if ((rc = dalloc(h, &h->S2, h->S_bytes))) return bail(rc);
+    } else if (h->fftp) {  // so does the plane pass; without the memory, cuFFT's plan in place
+        if (dalloc(h, &h->S2, h->S_bytes) != GABE_OK) {
+            h->S2 = nullptr;
+            h->fftp = false;
+            h->err.clear();
+        }
     } else if (h->evolve_gw && !(p->flags & GABE_FLAG_NO_OVERLAP)) {
         // optional: without it the GW chain simply runs in line
         if (dalloc(h, &h->S2, h->S_bytes) != GABE_OK) {
@@ -527,6 +553,7 @@ int gabe_create(const gabe_params *p, gabe_handle **out) {
         set_err(h, GABE_ERR_CUDA, "stream/event creation failed");
         return bail(GABE_ERR_CUDA);
     }
+    h->gt = h->fftp ? 2 : h->fftt ? 1 : 0;
     const size_t nblk_stencil = (size_t)h->grid.x * h->grid.y * h->grid.z;
     h->npartials = kNV * (nblk_stencil > 4096 ? nblk_stencil : 4096);
     if ((rc = dalloc(h, (void **)&h->partials, h->npartials * sizeof(double)))) return bail(rc);
@@ -671,7 +698,7 @@ int gabe_profile_steps(gabe_handle *h, int nsteps, double ms_out[4]) {
     return read_scalars(h, &sc);
 }
 
-// Transposed form: nreps full steps with events around each of its three launches.
+// Transposed and plane forms: nreps full steps with events around each of their three launches.
 static int profile_fftt_passes(gabe_handle *h, int nreps, double ms_out[3]) {
     std::vector<cudaEvent_t> ev((size_t)4 * nreps, nullptr);
     for (auto &x : ev) CK(h, cudaEventCreate(&x));
@@ -682,13 +709,21 @@ static int profile_fftt_passes(gabe_handle *h, int nreps, double ms_out[3]) {
         rc = sweep(h, MODE_A_GW, c, 0, 0);
         if (rc) break;
         cudaError_t ce = cudaEventRecord(e[0], h->stream);
-        if (ce == cudaSuccess) ce = fftt_rows_f32(h->N, static_cast<const float *>(h->S), h->S2, 2 * kSrc, &h->sc->status,
-                                                         h->stream);
+        const float *S = static_cast<const float *>(h->S);
+        float *S2 = static_cast<float *>(h->S2);
+        const size_t half = (size_t)kSrc * h->N * h->N * (h->N + 2);
+        unsigned int *st = &h->sc->status;
+        if (ce == cudaSuccess)
+            ce = h->fftp ? fftp_planes_f32(h->N, S, S2, kSrc * h->N, h->stream)
+                         : fftt_rows_f32(h->N, S, S2, 2 * kSrc, st, h->stream);
         if (ce == cudaSuccess) ce = cudaEventRecord(e[1], h->stream);
-        if (ce == cudaSuccess) ce = fftt_cols_f32(h->N, h->S2, h->S, 2 * kSrc, &h->sc->status, h->stream);
+        if (ce == cudaSuccess)
+            ce = h->fftp ? fftp_planes_f32(h->N, S + half, S2 + half, kSrc * h->N, h->stream)
+                         : fftt_cols_f32(h->N, h->S2, h->S, 2 * kSrc, st, h->stream);
         if (ce == cudaSuccess) ce = cudaEventRecord(e[2], h->stream);
         if (ce == cudaSuccess)
-            ce = fftt_ikspace_f32(h->N, h->S, h->G, h->sc, h->lc, 0, &h->sc->status, h->stream);
+            ce = h->fftp ? fftp_lines_f32(h->N, h->S2, h->G, h->sc, nullptr, 1, h->lc, 0, h->stream)
+                         : fftt_ikspace_f32(h->N, h->S, h->G, h->sc, h->lc, 0, st, h->stream);
         if (ce == cudaSuccess) ce = cudaEventRecord(e[3], h->stream);
         if (ce != cudaSuccess) {
             rc = set_err(h, GABE_ERR_CUDA, "profile launch: %s", cudaGetErrorString(ce));
@@ -716,7 +751,7 @@ static int profile_fftt_passes(gabe_handle *h, int nreps, double ms_out[3]) {
 int gabe_profile_fft_passes(gabe_handle *h, int nreps, double ms_out[3]) {
     if (!h || !ms_out || nreps < 1) return GABE_ERR_PARAM;
     if (!h->uploaded) return set_err(h, GABE_ERR_STATE, "profile before upload");
-    if (h->fftt) {
+    if (h->fftt || h->fftp) {
         CK(h, cudaSetDevice(h->dev));
         return profile_fftt_passes(h, nreps, ms_out);
     }
@@ -912,7 +947,7 @@ int gabe_spectra_raw(gabe_handle *h, double *sums, double *counts, int nbins, in
     b.nseries = ns;
     b.quirk = h->p.gw_spec_quirk;
     b.fix_zero = h->f32 ? 1 : 0;
-    b.gt = h->fftt ? 1 : 0;
+    b.gt = h->gt;
     b.zero_re[0] = h->lc.gridsize * s.fbar[0];
     b.zero_re[1] = h->lc.gridsize * s.fbar[1];
     const size_t smem = (size_t)h->nbins * (ns * 8 + 4);
@@ -1010,6 +1045,9 @@ int read_device(gabe_handle *h, FILE *f, void *dev, size_t bytes, std::vector<ch
         if (fread(bounce.data(), 1, n, f) != n) return set_err(h, GABE_ERR_PARAM, "checkpoint file is truncated");
         CK(h, cudaMemcpy(static_cast<char *>(dev) + o, bounce.data(), n, cudaMemcpyHostToDevice));
     }
+    // a copy from pageable memory may return before its last bytes have left the staging buffer, and the
+    // handle's stream does not wait for the default one
+    CK(h, cudaStreamSynchronize(nullptr));
     return GABE_OK;
 }
 
@@ -1017,7 +1055,7 @@ void fill_restart(const gabe_handle *h, gabe_restart_header *r) {
     std::memset(r, 0, sizeof(*r));
     std::memcpy(r->magic, GABE_RESTART_MAGIC, 8);
     r->precision = h->p.precision;
-    r->gw_layout = h->fftt ? 1 : 0;
+    r->gw_layout = h->gt;
     r->expansion = h->p.expansion;
     r->tile_shape = h->shape;
     r->tile_ci = h->ci;
@@ -1113,7 +1151,9 @@ int gabe_load_state(gabe_handle *h, const char *path, int *restored) {
     bool native = false;
     if (fseeko(fc.f, (off_t)(sizeof(hd) + payload), SEEK_SET) == 0 && fread(&r, sizeof(r), 1, fc.f) == 1 &&
         std::memcmp(r.magic, GABE_RESTART_MAGIC, 8) == 0) {
-        native = r.precision == want.precision && r.gw_layout == want.gw_layout && r.expansion == want.expansion &&
+        // amplitudes in another order (another transform form wrote the file) are reordered below
+        const bool orders = r.gw_layout == want.gw_layout || (h->f32 && r.gw_layout >= 0 && r.gw_layout <= 2);
+        native = r.precision == want.precision && orders && r.expansion == want.expansion &&
                  r.scalar_bytes == want.scalar_bytes && r.elem_bytes == want.elem_bytes &&
                  r.field_bytes == want.field_bytes && r.gw_bytes == want.gw_bytes && hd.gws == h->p.gws_on;
     }
@@ -1128,7 +1168,16 @@ int gabe_load_state(gabe_handle *h, const char *path, int *restored) {
         if ((rc = read_device(h, fc.f, h->X[0], (size_t)r.field_bytes, bounce)) ||
             (rc = read_device(h, fc.f, h->D[0], (size_t)r.field_bytes, bounce)))
             return rc;
-        if (r.gw_bytes && (rc = read_device(h, fc.f, h->G, (size_t)r.gw_bytes, bounce))) return rc;
+        if (r.gw_bytes && r.gw_layout == h->gt) {
+            if ((rc = read_device(h, fc.f, h->G, (size_t)r.gw_bytes, bounce))) return rc;
+        } else if (r.gw_bytes) {
+            const size_t one = (size_t)r.gw_bytes / 4;  // one amplitude array; S holds at least two field spectra
+            for (int p = 0; p < 4; p++) {
+                if ((rc = read_device(h, fc.f, h->S, one, bounce))) return rc;
+                CK(h, gw_reorder_f32(h->S, static_cast<char *>(h->G) + p * one, h->N, r.gw_layout, h->gt, h->stream));
+                CK(h, cudaStreamSynchronize(h->stream));
+            }
+        }
         CK(h, cudaMemcpy(h->sc, &sc, sizeof(sc), cudaMemcpyHostToDevice));
         h->cur = 0;
         h->e0_stale = r.e0_stale != 0;
@@ -1161,7 +1210,7 @@ int gabe_graph_active(const gabe_handle *h) {
 }
 
 int gabe_launches_per_step(const gabe_handle *h) {
-    return h ? (h->evolve_gw ? (h->own_fft ? 6 : h->fftt ? 5 : 3) : 2) : 0;
+    return h ? (h->evolve_gw ? (h->own_fft ? 6 : h->fftt || h->fftp ? 5 : 3) : 2) : 0;
 }
 
 }  // extern "C"

@@ -26,6 +26,9 @@ using namespace gabe;
 namespace {
 thread_local std::string g_ens_create_error;
 constexpr int kEnsBinBlocks = 32;  // binning blocks per lattice
+// Transformed planes of one batch of the plane transform: the batch size hardly matters (24 to 96 MB 632-637 ms
+// per 50 steps of the 256-lattice ensemble, 1 GB 639), so it is kept small; one stream instead of two 672.
+constexpr size_t kPlaneBatchBytes = (size_t)48 << 20;
 }  // namespace
 
 struct gabe_ensemble {
@@ -43,6 +46,9 @@ struct gabe_ensemble {
         Cplx<float> *G = nullptr;
         cufftHandle plan_src = 0, plan_ic = 0, plan_spec = 0;
         bool have_src = false, have_ic = false, have_spec = false;
+        bool plane = false;  // GW sources through the plane transform, `batch` lattices at a time
+        int batch = 0;
+        int *ids = nullptr;  // device: the group's lattices, in pool order
     };
     std::vector<Group> groups;
     std::vector<EnsLat> h_lat;
@@ -53,6 +59,11 @@ struct gabe_ensemble {
     unsigned int *d_lat_count = nullptr;
     DevScalars *d_sc = nullptr;
     int nkchunks = 0;
+    // the plane transform's batches alternate between two side streams, each with the transformed planes of one
+    cudaStream_t side[2] = {nullptr, nullptr};
+    cudaEvent_t ev_a = nullptr, ev_side[2] = {nullptr, nullptr};
+    float *T[2] = {nullptr, nullptr};
+    int gw_launches = 0; // plane transform and k-space launches per step
     void *fft_work = nullptr;
     double *d_m2 = nullptr, *d_sumsq = nullptr;
     double *d_part = nullptr, *d_log = nullptr, *d_logcnt = nullptr, *d_native = nullptr;
@@ -105,6 +116,8 @@ int ealloc(gabe_ensemble *e, void **p, size_t bytes) {
     return GABE_OK;
 }
 
+size_t lattice_M(int N) { return (size_t)N * N * (N / 2 + 1); }
+
 gabe_params lattice_params(const gabe_ensemble *e, int l) {
     gabe_params p;
     gabe_default_params(&p, e->N[l]);
@@ -125,7 +138,7 @@ int make_plans(gabe_ensemble *e) {
         long long n[3] = {N, N, N};
         const long long slot_r = N * N * 2 * nz, slot_c = N * N * nz;  // one source slot in reals / complex
         size_t w = 0;
-        if (e->gws) {
+        if (e->gws && !G.plane) {
             long long inem[3] = {N, N, 2 * nz}, onem[3] = {N, N, nz};
             ECF(e, cufftCreate(&G.plan_src));
             G.have_src = true;
@@ -204,11 +217,40 @@ int enqueue_step(gabe_ensemble *e, int cur) {
     int rc = sweep(e, e->gws ? MODE_A_GW : MODE_A, cur);
     if (rc) return rc;
     if (e->gws) {
-        for (auto &G : e->groups) ECF(e, cufftExecR2C(G.plan_src, (cufftReal *)G.S, (cufftComplex *)G.S));
-        ens_kspace_kernel<<<e->nkchunks, 256, 0, e->stream>>>(ens_args(e, cur));
-        ECK(e, cudaGetLastError());
+        // The GW chain reads what sweep A wrote (sources, DevScalars::gw) and nothing that sweep B writes: its
+        // batches run on the side streams beside sweep B, filling each other's last waves.
+        if (e->T[0]) {
+            ECK(e, cudaEventRecord(e->ev_a, e->stream));
+            for (int b = 0; b < 2; b++) ECK(e, cudaStreamWaitEvent(e->side[b], e->ev_a, 0));
+        }
+        int turn = 0;
+        for (auto &G : e->groups) {
+            if (!G.plane) {
+                ECF(e, cufftExecR2C(G.plan_src, (cufftReal *)G.S, (cufftComplex *)G.S));
+                continue;
+            }
+            const int ng = (int)G.lats.size();
+            const size_t slots = (size_t)2 * kSrc * G.N * G.N * (G.N + 2), M4 = 4 * lattice_M(G.N);
+            for (int l0 = 0; l0 < ng; l0 += G.batch, turn ^= 1) {
+                const int n = std::min(G.batch, ng - l0);
+                ECK(e, fftp_planes_f32(G.N, G.S + l0 * slots, e->T[turn], n * 2 * kSrc * G.N, e->side[turn]));
+                ECK(e, fftp_lines_f32(G.N, e->T[turn], G.G + l0 * M4, e->d_sc, G.ids + l0, n, e->h_lat[G.lats[0]].c, 0,
+                                      e->side[turn]));
+            }
+        }
+        if (e->nkchunks) {
+            ens_kspace_kernel<<<e->nkchunks, 256, 0, e->stream>>>(ens_args(e, cur));
+            ECK(e, cudaGetLastError());
+        }
     }
-    return sweep(e, MODE_B, cur);
+    int rc2 = sweep(e, MODE_B, cur);
+    if (rc2) return rc2;
+    if (e->gws && e->T[0])
+        for (int b = 0; b < 2; b++) {
+            ECK(e, cudaEventRecord(e->ev_side[b], e->side[b]));
+            ECK(e, cudaStreamWaitEvent(e->stream, e->ev_side[b], 0));
+        }
+    return GABE_OK;
 }
 
 int refresh_e0(gabe_ensemble *e) {
@@ -218,8 +260,6 @@ int refresh_e0(gabe_ensemble *e) {
     e->e0_stale = false;
     return GABE_OK;
 }
-
-size_t lattice_M(int N) { return (size_t)N * N * (N / 2 + 1); }
 
 }  // namespace
 
@@ -293,6 +333,35 @@ int gabe_ensemble_create(const gabe_ensemble_params *p, gabe_ensemble **out) {
         e->groups[gidx[e->N[l]]].lats.push_back(l);
     }
     int rc;
+    if (e->gws) {
+        // batches of the plane transform: the transformed planes of one (10 N^2 (N+2) floats per lattice) fit
+        // the L2 cache beside the sources streaming through it
+        size_t tmax = 0;
+        for (auto &G : e->groups) {
+            G.plane = fftp_supported(G.N);
+            if (!G.plane) continue;
+            const size_t one = (size_t)2 * kSrc * G.N * G.N * (G.N + 2) * sizeof(float);
+            G.batch = std::max<int>(1, (int)std::min<size_t>(G.lats.size(), kPlaneBatchBytes / one));
+            tmax = std::max(tmax, G.batch * one);
+            e->gw_launches += 2 * (int)((G.lats.size() + G.batch - 1) / G.batch);
+            if ((rc = ealloc(e, (void **)&G.ids, sizeof(int) * G.lats.size()))) return bail(rc);
+            if (cudaMemcpy(G.ids, G.lats.data(), sizeof(int) * G.lats.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+                cudaGetLastError();
+                eset(e, GABE_ERR_CUDA, "ensemble set-up copies failed");
+                return bail(GABE_ERR_CUDA);
+            }
+        }
+        for (int b = 0; tmax && b < 2; b++) {
+            if ((rc = ealloc(e, (void **)&e->T[b], tmax))) return bail(rc);
+            if (cudaStreamCreateWithFlags(&e->side[b], cudaStreamNonBlocking) != cudaSuccess ||
+                cudaEventCreateWithFlags(&e->ev_side[b], cudaEventDisableTiming) != cudaSuccess ||
+                (b == 0 && cudaEventCreateWithFlags(&e->ev_a, cudaEventDisableTiming) != cudaSuccess)) {
+                cudaGetLastError();
+                eset(e, GABE_ERR_CUDA, "stream/event creation failed");
+                return bail(GABE_ERR_CUDA);
+            }
+        }
+    }
     if ((rc = ealloc(e, (void **)&e->d_sc, sizeof(DevScalars) * e->nlat))) return bail(rc);
     e->h_lat.resize(e->nlat);
     for (auto &G : e->groups) {
@@ -316,6 +385,7 @@ int gabe_ensemble_create(const gabe_ensemble_params *p, gabe_ensemble **out) {
             }
             Lt.S = G.S + q * 2 * kSrc * slot_r;
             Lt.G = e->gws ? G.G + q * 4 * M : nullptr;
+            Lt.gt = G.plane ? 2 : 0;
             Lt.sc = e->d_sc + l;
             Lt.N = G.N;
             Lt.seed = e->seed[l];
@@ -335,14 +405,15 @@ int gabe_ensemble_create(const gabe_ensemble_params *p, gabe_ensemble **out) {
                 for (int k0 = 0; k0 < n; k0 += TK) items.push_back({l, e->shape[l], j0, k0, i0, std::min(i0 + c, n)});
         Lt.nitems = (int)items.size() - Lt.first_item;
         Lt.first_kchunk = (int)nkc;
-        nkc += (lattice_M(n) + kEnsKChunk - 1) / kEnsKChunk;
+        if (Lt.gt == 0) nkc += (lattice_M(n) + kEnsKChunk - 1) / kEnsKChunk;
     }
     if (items.size() > (size_t)INT32_MAX || nkc > (size_t)INT32_MAX) {
         eset(e, GABE_ERR_PARAM, "ensemble too large for one launch");
         return bail(GABE_ERR_PARAM);
     }
     e->nitems = (int)items.size();
-    e->nkchunks = (int)nkc;
+    e->nkchunks = e->gws ? (int)nkc : 0;
+    e->gw_launches += e->nkchunks ? 1 : 0;
     if ((rc = ealloc(e, (void **)&e->d_lat, sizeof(EnsLat) * e->nlat))) return bail(rc);
     if ((rc = ealloc(e, (void **)&e->d_items, sizeof(EnsItem) * e->nitems))) return bail(rc);
     // per-item partial sums; also the scratch of the upload's mean reduction (256 blocks)
@@ -381,8 +452,13 @@ int gabe_ensemble_destroy(gabe_ensemble *e) {
     if (!e) return GABE_OK;
     cudaSetDevice(e->dev);
     if (e->stream) cudaStreamSynchronize(e->stream);
-    for (int i = 0; i < 2; i++)
+    for (int i = 0; i < 2; i++) {
+        if (e->side[i]) cudaStreamSynchronize(e->side[i]);
         if (e->graph[i]) cudaGraphExecDestroy(e->graph[i]);
+        if (e->ev_side[i]) cudaEventDestroy(e->ev_side[i]);
+        if (e->side[i]) cudaStreamDestroy(e->side[i]);
+    }
+    if (e->ev_a) cudaEventDestroy(e->ev_a);
     for (auto &G : e->groups) {
         if (G.have_src) cufftDestroy(G.plan_src);
         if (G.have_ic) cufftDestroy(G.plan_ic);
@@ -618,7 +694,7 @@ int gabe_ensemble_download(gabe_ensemble *e, int lat, double *field0, double *df
         if (!gdst[w] || !Lt.G) continue;
         for (size_t m0 = 0; m0 < M; m0 += chunk) {
             const size_t cnt = (M - m0) < chunk ? (M - m0) : chunk;
-            ECK(e, gw_unpack_f32(Lt.G, cnt, m0, Lt.N, M, w, stage, 0, e->stream));
+            ECK(e, gw_unpack_f32(Lt.G, cnt, m0, Lt.N, M, w, stage, Lt.gt, e->stream));
             for (int q = 0; q < 12; q++)
                 ECK(e, cudaMemcpyAsync(gdst[w] + (size_t)q * M + m0, stage + (size_t)q * cnt, cnt * 8,
                                        cudaMemcpyDeviceToHost, e->stream));
@@ -634,7 +710,7 @@ size_t gabe_ensemble_device_bytes(const gabe_ensemble *e) { return e ? e->dev_by
 
 void *gabe_ensemble_stream(const gabe_ensemble *e) { return e ? (void *)e->stream : nullptr; }
 
-int gabe_ensemble_launches_per_step(const gabe_ensemble *e) { return e ? (e->gws ? 3 : 2) : 0; }
+int gabe_ensemble_launches_per_step(const gabe_ensemble *e) { return e ? 2 + e->gw_launches : 0; }
 
 int gabe_ensemble_graph_active(const gabe_ensemble *e) {
     if (!e) return GABE_ERR_PARAM * -1;

@@ -10,10 +10,13 @@
 //     32x16 or 16x16 sites); per-item partial sums are combined by the block
 //     that finishes the last item of a lattice, in item order, so every
 //     lattice gets its own Friedmann update without a grid-wide barrier;
-//   * the GW transforms are one cuFFT call per lattice size (batch = 10 x
-//     lattices of that size, sources of a size group contiguous);
-//   * the k-space update is one kernel over the half spectra of all
-//     lattices, in chunks of one lattice per block.
+//   * the GW transforms and the k-space update are the plane transform's two
+//     launches (fftp.cuh) per batch of lattices of one size, a batch's
+//     transformed planes small enough to stay in L2 between them;
+//   * at sizes the plane transform does not take: one cuFFT call per lattice
+//     size (batch = 10 x lattices of that size, sources of a size group
+//     contiguous) and one k-space kernel over those lattices, in chunks of
+//     one lattice per block.
 // The initial state is drawn on the device with the reference's randInit
 // distribution (g2init.cpp:68-189) from a counter-based generator (Philox
 // 4x32-10, Salmon et al., SC'11), so it matches the reference in
@@ -34,7 +37,8 @@ struct EnsLat {
     float *S;            // [10][N][N][N+2] sources / [..][N][N][N/2+1] spectra
     Cplx<float> *G;      // [4][M] h+, hx, l+, lx
     DevScalars *sc;
-    int first_kchunk;    // first block of the k-space update that takes this lattice
+    int gt;              // order of G (g_index): 2 with the plane transform, 0 with cuFFT's
+    int first_kchunk;    // first block of the k-space update that takes this lattice (cuFFT's sizes only)
     int first_item, nitems;
     int N;
     unsigned long long seed;  // IC: counter-based generator key
@@ -299,7 +303,7 @@ __global__ void __launch_bounds__(256) ens_bin_kernel(EnsBinArgs a) {
     const int N = E.N;
     const Cplx<float> *F = reinterpret_cast<const Cplx<float> *>(E.S);
     const double zre[2] = {E.c.gridsize * E.sc->fbar[0], E.c.gridsize * E.sc->fbar[1]};
-    bin_points<float>(F, E.G, N, N, 0, 0, a.quirk, zre, nb, hs, hc, blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32,
+    bin_points<float>(F, E.G, N, N, 0, E.gt, a.quirk, zre, nb, hs, hc, blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32,
                       a.nblk * (blockDim.x / 32));
     __syncthreads();
     double *ps = a.part + ((size_t)blockIdx.y * a.nblk + blockIdx.x) * 3 * nb;

@@ -434,7 +434,7 @@ __global__ void __launch_bounds__(T, MINB) ikspace_kernel(IkArgs a) {
 #pragma unroll
             for (int p = 0; p < 4; p++) g[p] = {gv[r][p].x, gv[r][p].y};
             const int px = kx <= N / 2 ? kx : kx - N;
-            kspace_update_vals<float, true>(kc, px, py, kz, s, g);
+            kspace_update_vals<float, POL_FLOAT>(kc, px, py, kz, s, g);
 #pragma unroll
             for (int p = 0; p < 4; p++) __stcs(gl + p * M + kx, make_float2(g[p].re, g[p].im));
         }

@@ -97,6 +97,12 @@ cudaError_t gw_unpack_f32(const void *G, size_t cnt, size_t m0, int N, size_t M,
     return cudaGetLastError();
 }
 
+cudaError_t gw_reorder_f32(const void *from, void *to, int N, int gt_from, int gt_to, cudaStream_t s) {
+    gw_reorder_kernel<float><<<4 * 148, 256, 0, s>>>(static_cast<const Cplx<float> *>(from), static_cast<Cplx<float> *>(to),
+                                                     N, gt_from, gt_to);
+    return cudaGetLastError();
+}
+
 cudaError_t bins_f32(const BinArgs &a, const Launch &l) {
     bin_kernel<float><<<l.grid, l.block, l.smem, l.stream>>>(a);
     return cudaGetLastError();

@@ -114,24 +114,77 @@ __device__ __forceinline__ KsCoef<T> ks_coef(const LatticeConsts &c, const doubl
     return k;
 }
 
+// How a kernel forms the polarization tensors of a k-point.
+enum PolForm {
+    POL_DOUBLE = 0,   // FP64 unit vectors (pol_tensors)
+    POL_FLOAT = 1,    // FP32 unit vectors (pol_tensors32)
+    POL_RATIONAL = 2  // FP64 from the integer components, without unit vectors
+};
+
+// Weights of (S11, S12, S13, S22, S23) in eps:S/2 for a symmetric traceless
+// S, S33 = -S11 - S22, in the basis of pol_tensors.  With n the integer wave
+// vector, r its smallest component's axis, u = |n|^2 e_r - n_r n and
+// v = n x e_r:  e1 = u / (|n| s), e2 = v / s, s^2 = |n|^2 - n_r^2, so that
+//   eps+ = 2 u u / (|n|^2 s^2) - 1 + n n / |n|^2,  epsx = (u v + v u) / (|n| s^2):
+// products of integers, exact in FP64, one division and one square root,
+// about a third of pol_tensors' instructions.
+template <typename T>
+__device__ __forceinline__ void pol_weights(int px, int py, int pz, T (&wp)[5], T (&wx)[5]) {
+    const int ax = abs(px), ay = abs(py), az = abs(pz);
+    const int r = (ax <= ay && ax <= az) ? 0 : (ay <= az ? 1 : 2);
+    const double x = px, y = py, z = pz;
+    const double m2 = x * x + y * y + z * z;
+    const double nr = r == 0 ? x : (r == 1 ? y : z);
+    const double s2 = m2 - nr * nr;
+    const double inv = 1.0 / (m2 * s2);  // 1 / (|n|^2 s^2)
+    const double is = s2 * inv, two = 2.0 * inv, ix = sqrt(m2) * inv;
+    const double ux = (r == 0 ? m2 : 0.0) - nr * x, uy = (r == 1 ? m2 : 0.0) - nr * y, uz = (r == 2 ? m2 : 0.0) - nr * z;
+    const double vx = r == 0 ? 0.0 : (r == 1 ? -z : y), vy = r == 0 ? z : (r == 1 ? 0.0 : -x),
+                 vz = r == 0 ? -y : (r == 1 ? x : 0.0);
+    const double p0 = two * ux * ux + x * x * is, p3 = two * uy * uy + y * y * is, p5 = two * uz * uz + z * z * is;
+    wp[0] = (T)(0.5 * (p0 - p5));
+    wp[1] = (T)(two * ux * uy + x * y * is);
+    wp[2] = (T)(two * ux * uz + x * z * is);
+    wp[3] = (T)(0.5 * (p3 - p5));
+    wp[4] = (T)(two * uy * uz + y * z * is);
+    const double x5 = uz * vz;
+    wx[0] = (T)(ix * (ux * vx - x5));
+    wx[1] = (T)(ix * (ux * vy + uy * vx));
+    wx[2] = (T)(ix * (ux * vz + uz * vx));
+    wx[3] = (T)(ix * (uy * vy - x5));
+    wx[4] = (T)(ix * (uy * vz + uz * vy));
+}
+
 // Both RK2 stages of the amplitudes g[4] (h+, hx, l+, lx) of the k-point
 // with integer wave vector (px, py, kzi), driven by its transformed
 // sources s[10] (stage-0 11,12,13,22,23, then stage 1); g is updated in
 // place.  k = 0 has no TT part and is left as it is.
-// P: precision of the polarization tensors (double, or float for POL32).
-template <typename T, bool POL32 = false>
+template <typename T, int POL = POL_DOUBLE>
 __device__ __forceinline__ void kspace_update_vals(const KsCoef<T> &kc, int px, int py, int kzi, const Cplx<T> (&s)[10],
                                                    Cplx<T> (&g)[4]) {
     const double m2 = ((double)px * px + (double)py * py) + (double)kzi * kzi;
     if (m2 == 0.0) return;  // no TT mode at k = 0; its amplitudes stay zero
-    using P = typename std::conditional<POL32, float, double>::type;
-    P ep[6], ex[6];
-    if constexpr (POL32) pol_tensors32(px, py, kzi, ep, ex);
-    else pol_tensors(px, py, kzi, ep, ex);
-    // weights of (S11, S12, S13, S22, S23) in eps:S/2 with S33 = -S11-S22
-    const P half = (P)0.5;
-    const T wp[5] = {(T)(half * (ep[0] - ep[5])), (T)ep[1], (T)ep[2], (T)(half * (ep[3] - ep[5])), (T)ep[4]};
-    const T wx[5] = {(T)(half * (ex[0] - ex[5])), (T)ex[1], (T)ex[2], (T)(half * (ex[3] - ex[5])), (T)ex[4]};
+    T wp[5], wx[5];
+    if constexpr (POL == POL_RATIONAL) {
+        pol_weights<T>(px, py, kzi, wp, wx);
+    } else {
+        using P = typename std::conditional<POL == POL_FLOAT, float, double>::type;
+        P ep[6], ex[6];
+        if constexpr (POL == POL_FLOAT) pol_tensors32(px, py, kzi, ep, ex);
+        else pol_tensors(px, py, kzi, ep, ex);
+        // weights of (S11, S12, S13, S22, S23) in eps:S/2 with S33 = -S11-S22
+        const P half = (P)0.5;
+        wp[0] = (T)(half * (ep[0] - ep[5]));
+        wx[0] = (T)(half * (ex[0] - ex[5]));
+        wp[3] = (T)(half * (ep[3] - ep[5]));
+        wx[3] = (T)(half * (ex[3] - ex[5]));
+#pragma unroll
+        for (int q = 1; q < 5; q++) {
+            if (q == 3) continue;
+            wp[q] = (T)ep[q];
+            wx[q] = (T)ex[q];
+        }
+    }
     const T kk0 = (T)(m2 * kc.norm0), kk1 = (T)(m2 * kc.norm1);
     T Tp[2][2][2];  // [stage][pol][re/im], already times 2 (8 pi/a^2) dx^3
 #pragma unroll
@@ -206,10 +259,14 @@ __global__ void __launch_bounds__(256) kspace_kernel(KspaceArgs args) {
 }
 
 // Element of the amplitude arrays that holds k-point (i, j, kz) of the half
-// spectrum: [i][j][kz] (the library r2c's order), or [kz][j][i] for the
-// transposed transform of fftt.cuh (gt = 1).
+// spectrum: gt = 0 [i][j][kz] (the library r2c's order), 1 [kz][j][i] (the
+// transposed transform of fftt.cuh), 2 [x / 8][i][x % 8] with
+// x = j (N/2+1) + kz (the plane transform of fftp.cuh).
 __host__ __device__ inline size_t g_index(int i, int j, int kz, int N, int gt) {
-    return gt ? ((size_t)kz * N + j) * N + i : ((size_t)i * N + j) * (N / 2 + 1) + kz;
+    if (gt == 1) return ((size_t)kz * N + j) * N + i;
+    if (gt == 0) return ((size_t)i * N + j) * (N / 2 + 1) + kz;
+    const int x = j * (N / 2 + 1) + kz;
+    return ((size_t)(x >> 3) * N + i) * 8 + (x & 7);
 }
 
 // ---------------------------------------------------------------------------
@@ -296,6 +353,17 @@ __global__ void gw_unpack_kernel(const Cplx<T> *G, size_t cnt, size_t m0, int N,
             dst[(size_t)(2 * c6) * cnt + q] = ep[c6] * (double)ap.re + ex[c6] * (double)ax.re;
             dst[(size_t)(2 * c6 + 1) * cnt + q] = ep[c6] * (double)ap.im + ex[c6] * (double)ax.im;
         }
+    }
+}
+
+// One amplitude array from one order to another.
+template <typename T>
+__global__ void gw_reorder_kernel(const Cplx<T> *from, Cplx<T> *to, int N, int gt_from, int gt_to) {
+    const int nz = N / 2 + 1;
+    const size_t M = (size_t)N * N * nz;
+    for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < M; q += (size_t)gridDim.x * blockDim.x) {
+        const int kz = (int)(q % nz), j = (int)(q / nz % N), i = (int)(q / nz / N);
+        to[g_index(i, j, kz, N, gt_to)] = from[g_index(i, j, kz, N, gt_from)];
     }
 }
 

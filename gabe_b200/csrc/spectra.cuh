@@ -37,7 +37,7 @@ struct BinArgs {
     int fix_zero;
     // a slab's k-points (slab.cu): F and G hold [..][N][m][N/2+1] with ky = y0 + y; m = 0: all of them
     int m, y0;
-    int gt;                 // G in the transposed order [4][kz][ky][kx] (fftt.cuh); whole lattices only
+    int gt;                 // order of G (g_index); 1 and 2 for whole lattices only
 };
 
 // |n| of an integer wave vector, rounded down.  n2 <= 3 (N/2)^2 < 2^24 is
@@ -146,8 +146,9 @@ __device__ __forceinline__ void bin_points(const Cplx<T> *F, const Cplx<T> *G, i
                         if (at == 0 && y0 == 0) re += zero_re[f];  // k = 0
                         p[f] += re * re + im * im;
                     }
-                    if (G && !gt) {
-                        const size_t src = (quirk && kz == 0) ? at + (size_t)(N / 2) : at;
+                    if (G && gt != 1) {
+                        const int lz = (quirk && kz == 0) ? N / 2 : kz;
+                        const size_t src = gt == 2 ? g_index(si ? N - i : i, sj ? N - y : y, lz, N, 2) : at + (lz - kz);
                         g += l_power(G[2 * M + src], G[3 * M + src]);
                     }
                 }
@@ -163,9 +164,9 @@ __device__ __forceinline__ void bin_points(const Cplx<T> *F, const Cplx<T> *G, i
         if (r.head && ok) atomicAdd(&hc[r.bin], c);
         bin_add(r, wt * p[0], hs);
         bin_add(r, wt * p[1], hs + nb);
-        if (G && !gt) bin_add(r, wt * g, hs + 2 * nb);
+        if (G && gt != 1) bin_add(r, wt * g, hs + 2 * nb);
     }
-    if (!G || !gt) return;
+    if (!G || gt != 1) return;
     // amplitudes [kz][ky][kx] in their own order
     for (WarpWalk w(first, count, nz, nz); w.any(); w.next()) {
         const bool ok = w.valid();

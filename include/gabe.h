@@ -71,21 +71,24 @@ enum gabe_flags {
                                  instead of overlapping the next field sweeps (saves 10 N^2(N+2)
                                  words of device memory).  With the library's 3-D FFT the chain runs
                                  in line anyway and the second buffer is the target of its column
-                                 passes (out of place, faster); this flag makes them in place */
+                                 passes (out of place, faster); this flag makes them in place.  The
+                                 transposed and plane transforms need the second buffer in any case */
     GABE_FLAG_OWN_FFT = 16,     /* FP32 with N in {64, 128, 256, 512}: transform the GW sources with the
                                    library's in-layout three-pass 3-D r2c (the layout of a library r2c)
                                    followed by the separate k-space pass, instead of the default */
-    GABE_FLAG_CUFFT_3D = 64,    /* FP32 at N in {128, 256, 512}: cuFFT's 3-D plan and the separate k-space
-                                   pass instead of the default transposed transform (cuFFT's plan is the
-                                   default at every other size and for FP64) */
+    GABE_FLAG_CUFFT_3D = 64,    /* FP32: cuFFT's 3-D plan and the separate k-space pass instead of the library's
+                                   default transform.  That is the plane transform (whole (j, k) planes
+                                   in shared memory, lines along i fused with the k-space update) at
+                                   multiples of 16 up to 160 other than 64, the transposed one at 256 and
+                                   512; cuFFT's plan is the default at every other size and for FP64 */
     GABE_FLAG_TRANSPOSED_FFT = 128 /* FP32 with N in {64, 128, 256, 512}: the library's transposed three-pass
                                    transform -- rows along k, then along j, each written transposed so
                                    that every pass reads whole contiguous lines (bulk copies), and the
                                    pass along i fused with the TT projection and h/l update, so the
                                    transformed sources are never written back.  The default for FP32 at
-                                   N in {128, 256, 512} (the fastest form measured there on B200; a tie
-                                   with cuFFT's plan at 64); needs the second source buffer whatever
-                                   GABE_FLAG_NO_OVERLAP says */
+                                   N in {256, 512} (the fastest form measured there on B200; the plane
+                                   transform is ahead by 4 % at 128, cuFFT's plan ties at 64); needs the
+                                   second source buffer whatever GABE_FLAG_NO_OVERLAP says */
 };
 
 /* Run-time form of the g2parameters.h knobs that the hot path reads.  Two
@@ -142,14 +145,16 @@ int gabe_step(gabe_handle *h, int nsteps);
  * state advances by nsteps.  Measurement hook; no reference counterpart. */
 int gabe_profile_steps(gabe_handle *h, int nsteps, double ms_out[4]);
 
-/* For a handle whose GW sources go through the library's 3-D FFT (FP32 at
- * N = 512 by default, or GABE_FLAG_OWN_FFT): runs its three passes nreps
+/* For a handle whose GW sources go through the library's 3-D FFT
+ * (GABE_FLAG_OWN_FFT): runs its three passes nreps
  * times on the source buffer (in place; the next step rewrites the
  * sources) with CUDA events between them and returns the mean milliseconds
  * of {rows along k, pass along j, pass along i}.  With
- * GABE_FLAG_TRANSPOSED_FFT: runs nreps full steps (the state advances) with
+ * the transposed transform: runs nreps full steps (the state advances) with
  * events around the transform's launches and returns {rows along k, pass
- * along j, pass along i fused with the k-space update}.  Other handles:
+ * along j, pass along i fused with the k-space update}.  With the plane
+ * transform likewise {planes of the stage-0 sources, planes of the stage-1
+ * sources, lines along i fused with the k-space update}.  Other handles:
  * GABE_ERR_STATE.  Measurement hook; no reference counterpart. */
 int gabe_profile_fft_passes(gabe_handle *h, int nreps, double ms_out[3]);
 
@@ -190,10 +195,11 @@ int gabe_download_state(gabe_handle *h, double *field0, double *dfield0, double 
 int gabe_save_state(gabe_handle *h, const char *path);
 
 /* Loads a gabe_dump.h file written for this handle's N, L, dt and model.
- * If it carries a restart block of the same precision, amplitude layout and
- * expansion type (a gabe_save_state file of an equal handle), that block
- * becomes the state and the run continues bit for bit (with the same tile
- * plan; *restored = 1).  Otherwise its FP64 arrays are uploaded as
+ * If it carries a restart block of the same precision and expansion type (a
+ * gabe_save_state file of an equal handle), that block becomes the state and
+ * the run continues bit for bit (with the same tile plan and transform form;
+ * *restored = 1; FP32 amplitudes written by another transform form are
+ * brought into this handle's order).  Otherwise its FP64 arrays are uploaded as
  * gabe_upload_state does (*restored = 0): e.g. the dumps of the reference
  * harness.  restored may be NULL.  A load that fails after it began to
  * overwrite the device state leaves the handle without a state, as a failed

@@ -60,7 +60,17 @@ __device__ __forceinline__ float silu(float z) { return z * sigmoid(z); }
 // second special-function operation measured slower (225 us): the
 // epilogue is bound by issue as much as by that pipe.  z -> -inf gives 0,
 // z -> +inf gives z.
-__device__ __forceinline__ float silu_fast(float z) { return __fdividef(z, 1.f + __expf(-z)); }
+// Written with the flush-to-zero forms of the two operations: the plain
+// intrinsics guard against subnormal operands and results with three more
+// instructions each, which cannot matter here (1 + exp(-z) >= 1, and a
+// flushed exponential adds nothing to 1; a flushed reciprocal is the 0 that
+// the division intrinsic gives for such divisors).
+__device__ __forceinline__ float silu_fast(float z) {
+    float e, r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(z * -1.4426950408889634f));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + e));
+    return z * r;
+}
 __device__ __forceinline__ float dsilu(float z) {
     const float s = sigmoid(z);
     return s * (1.f + z * (1.f - s));
@@ -645,6 +655,429 @@ __global__ void __launch_bounds__(NT, 1)
 
 }  // namespace t5
 
+// ---------------------------------------------------------------------------
+// The whole forward in one launch, for networks whose layers all take the
+// tcgen05 form above and the first-layer kernel: the activations of a tile of
+// 128 rows stay in shared memory from the first layer to the last, so HBM
+// sees the inputs and the outputs only (layer by layer, each hidden
+// activation crosses it twice: 4.3 GB of 5.1 at 1M rows).
+//
+// One persistent CTA per SM takes groups of two tiles (one where there are
+// fewer tiles than SMs): per tile its activations (K/64 slices of 128 x 64
+// BF16, 128-byte swizzle, as the MMA reads them) and a 256-column TMEM
+// accumulator, and one ring of 32 KB weight slots (up to 256 output columns x
+// 64 inputs) that streams each layer's weights from L2 once per tile.
+//   warp 0 (one thread)  tiled TMA loads of the weight slots, as far ahead
+//                        as the ring allows,
+//   warp 1 (one thread)  per layer and tile: the MMAs,
+//   warps 2-17           first layer on FMA, then per layer and tile bias +
+//                        SiLU of 32 x 32 blocks, in the old activations'
+//                        place (the tile's MMAs have completed), then the
+//                        output layer's blocks staged there and stored by TMA.
+// One tile's MMAs and weight loads run under the other's SiLU, which needs the
+// special-function pipe twice per value: 0.48 ms for 1M rows x 4 x 256
+// values at 1.9 GHz, four times what the tensor pipe needs.  A tile's output
+// layer is followed by the first layer of the next group's tile, so that the
+// other tile's MMAs have SiLU to run under there too.
+// Results are those of the layer-by-layer kernels bit for bit: the same
+// products in the same K order, the same epilogue arithmetic.
+// Measured (1M rows, default network): 0.80 ms against 1.02 for the five
+// launches; 41 rows 27 us a call against 47.  What set the pace on the way
+// there, read from clock stamps: divisions and remainders in the two issuing
+// threads (1000 cycles per weight slot beside 16 busy warps; 1.2 ms), 16 KB
+// slots (twice the waits and commits of 32 KB ones), a first layer by a lane
+// per row.  What is left: a hidden layer's SiLU takes 4.2-4.9k cycles per tile
+// (4.1k by the special-function pipe), the first layer's 8-9k.
+// Waits are bounded as in the kernel above.
+// ---------------------------------------------------------------------------
+namespace t6 {
+
+using gabe::tma::mbar_wait;
+using t5::BK;
+using t5::BM;
+using t5::pack_bf16;
+
+constexpr int kEpiWarps = 16, kThreadsPerCta = 64 + 32 * kEpiWarps;
+constexpr int kSlotBytes = 256 * BK * 2;  // up to 256 output columns x 64 inputs
+constexpr int kMaxSlots = 8;
+constexpr int kMaxLayers = 17;
+constexpr int kBlockBytes = 32 * 32 * 4;  // one staged FP32 output block
+constexpr uint32_t kCols = 256;           // TMEM columns per tile
+
+struct Args {
+    int M, width, n_in, n_out, nl, slots, tiles, box;  // tiles per group (1 or 2), rows per weight load
+    const float *x, *W0;
+    const float *bias[kMaxLayers];
+    int rowoff[kMaxLayers];  // first row of layer l in the stacked transposed weights
+    bf16 *H, *Z;             // KEEP: activations of hidden layer l at + l * keep_stride
+    long long keep_stride;
+    unsigned int *status;
+};
+
+// one tile's activations (also the staging area of its output blocks)
+__host__ __device__ inline size_t act_bytes(int width) {
+    const size_t a = (size_t)(width / BK) * BM * BK * 2, stage = (size_t)kEpiWarps * kBlockBytes;
+    return a < stage ? stage : a;
+}
+__host__ __device__ inline size_t smem_bytes(int width, int slots) {
+    return 1024 + 2 * act_bytes(width) + (size_t)slots * kSlotBytes + 256;
+}
+
+// Row `row` of the activations: 16-byte unit u of the 32 columns from col0 (a multiple of 32).
+__device__ __forceinline__ uint4 *act_unit(unsigned char *act, int row, int col0, int u) {
+    const int kb = col0 / BK, unit = (col0 % BK) / 8 + u;
+    return reinterpret_cast<uint4 *>(act + (size_t)kb * BM * BK * 2 + (row >> 3) * 1024 + (row & 7) * 128 +
+                                     ((unit ^ (row & 7)) << 4));
+}
+
+// Packed FP32 pairs: one issue slot for two values, each rounded as the scalar operation rounds it.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;"
+        : "=l"(reinterpret_cast<uint64_t &>(r))
+        : "l"(reinterpret_cast<uint64_t &>(a)), "l"(reinterpret_cast<uint64_t &>(b)),
+          "l"(reinterpret_cast<uint64_t &>(c)));
+    return r;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 r;
+    asm("add.rn.f32x2 %0, %1, %2;"
+        : "=l"(reinterpret_cast<uint64_t &>(r))
+        : "l"(reinterpret_cast<uint64_t &>(a)), "l"(reinterpret_cast<uint64_t &>(b)));
+    return r;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    float2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;"
+        : "=l"(reinterpret_cast<uint64_t &>(r))
+        : "l"(reinterpret_cast<uint64_t &>(a)), "l"(reinterpret_cast<uint64_t &>(b)));
+    return r;
+}
+// silu_fast of a pair
+__device__ __forceinline__ float2 silu2(float2 z) {
+    const float2 t = mul2(z, make_float2(-1.4426950408889634f, -1.4426950408889634f));
+    float2 e, r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.x) : "f"(t.x));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.y) : "f"(t.y));
+    e = add2(e, make_float2(1.f, 1.f));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(e.x));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(e.y));
+    return mul2(z, r);
+}
+
+// v += b, 32 values read by every lane (cached in L1)
+__device__ __forceinline__ void add_bias(float2 (&v)[16], const float *b) {
+    const float4 *bq = reinterpret_cast<const float4 *>(b);
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+        const float4 bb = __ldg(bq + u);
+        v[2 * u] = add2(v[2 * u], make_float2(bb.x, bb.y));
+        v[2 * u + 1] = add2(v[2 * u + 1], make_float2(bb.z, bb.w));
+    }
+}
+// This lane's row of 32 accumulator columns.
+__device__ __forceinline__ void load_block(uint32_t taddr, float2 (&v)[16]) {
+    float f[32];
+    gabe::umma::tmem_ld32(taddr, f);
+#pragma unroll
+    for (int j = 0; j < 16; j++) v[j] = make_float2(f[2 * j], f[2 * j + 1]);
+}
+
+// KEEP: also store the hidden layers' activations and pre-activations (training).
+// NIN: at least the number of inputs (4 or 8: weights a lane holds in the first layer).
+template <bool KEEP, int NIN>
+__global__ void __launch_bounds__(kThreadsPerCta, 1)
+    mlp_kernel(const __grid_constant__ CUtensorMap mapW, const __grid_constant__ CUtensorMap mapY,
+               const __grid_constant__ Args g) {
+    namespace tma = gabe::tma;
+    namespace umma = gabe::umma;
+    extern __shared__ unsigned char smraw[];
+    const uint32_t s0 = tma::saddr(smraw);
+    unsigned char *sm = smraw + (((s0 + 1023u) & ~1023u) - s0);
+    const int W = g.width, KB = W / BK, S = g.slots, nl = g.nl;
+    unsigned char *acts = sm;
+    const size_t AB = act_bytes(W);
+    unsigned char *ring = sm + 2 * AB;
+    uint64_t *wfull = reinterpret_cast<uint64_t *>(ring + (size_t)S * kSlotBytes);
+    uint64_t *wempty = wfull + kMaxSlots, *act = wempty + kMaxSlots, *dfull = act + 2, *sfree = dfull + 2,
+             *done = sfree + 2;  // act, dfull, sfree: one per tile
+    uint32_t *tbase_s = reinterpret_cast<uint32_t *>(done + 1);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rows_per_group = g.tiles * BM, ngroups = (g.M + rows_per_group - 1) / rows_per_group;
+    // tiles of group grp that hold rows
+    auto tiles_of = [&](int grp) { return g.tiles == 2 && (long long)grp * rows_per_group + BM < g.M ? 2 : 1; };
+    auto width_of = [&](int l) { return l + 1 == nl ? g.n_out : W; };
+
+    if (tid == 0) {
+        for (int s = 0; s < S; s++) {
+            tma::mbar_init(&wfull[s], 1);
+            tma::mbar_init(&wempty[s], 1);
+        }
+        for (int t = 0; t < 2; t++) {
+            tma::mbar_init(&act[t], 32 * kEpiWarps);
+            tma::mbar_init(&dfull[t], 1);
+            tma::mbar_init(&sfree[t], kEpiWarps);
+        }
+        tma::mbar_init(done, 1);
+        tma::fence_barrier_init();
+    }
+    if (warp == 1) umma::tmem_alloc(tbase_s, 2 * kCols);
+    umma::fence_before();
+    __syncthreads();
+    umma::fence_after();
+    const uint32_t tbase = *tbase_s;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int fills[kMaxSlots];
+            for (int s = 0; s < kMaxSlots; s++) fills[s] = 0;
+            int s = 0;
+            uint32_t phase = 1;  // parity of wempty[s] to wait for; flips as the ring wraps
+            bool ok = true;
+            for (int grp = blockIdx.x; ok && grp < ngroups; grp += gridDim.x) {
+                const int nt = tiles_of(grp);
+                for (int l = 1; ok && l < nl; l++) {
+                    const int y0 = g.rowoff[l], rows = width_of(l);
+                    for (int t = 0; ok && t < nt; t++)
+                        for (int x = 0; x < W; x += BK) {
+                            if (!mbar_wait(&wempty[s], phase, g.status)) {
+                                ok = false;
+                                break;
+                            }
+                            fills[s]++;
+                            tma::mbar_arrive_expect(&wfull[s], (uint32_t)rows * 128);
+                            unsigned char *dst = ring + (size_t)s * kSlotBytes;
+                            for (int r = 0; r < rows; r += g.box) umma::load_2d(dst + r * 128, &mapW, x, y0 + r, &wfull[s]);
+                            if (++s == S) {
+                                s = 0;
+                                phase ^= 1;
+                            }
+                        }
+                }
+            }
+            // every load issued has landed before the block may exit
+            tma::drain(wfull, fills, S, g.status);
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            bool ok = true;
+            // one thread issues everything, beside 16 busy warps: no divisions, descriptors by addition
+            int s = 0;
+            uint32_t phase = 0, pact = 0;  // parities of wfull[s], and of act[t] in bit t
+            const uint64_t da0 = umma::desc_k128(tma::saddr(acts)), db0 = umma::desc_k128(tma::saddr(ring));
+            const uint64_t da_tile = AB >> 4, da_kb = (BM * BK * 2) >> 4, db_slot = kSlotBytes >> 4;  // in 16-byte units
+            for (int grp = blockIdx.x; ok && grp < ngroups; grp += gridDim.x) {
+                const int nt = tiles_of(grp);
+                for (int l = 1; ok && l < nl; l++) {
+                    const uint32_t idesc = umma::idesc_bf16(BM, width_of(l));
+                    for (int t = 0; ok && t < nt; t++) {
+                        if (!(ok = mbar_wait(&act[t], (pact >> t) & 1u, g.status))) break;
+                        pact ^= 1u << t;
+                        umma::fence_after();
+                        const uint32_t d = tbase + (uint32_t)t * kCols;
+                        uint64_t da = da0 + (t ? da_tile : 0);
+                        for (int kb = 0; kb < KB; kb++, da += da_kb) {
+                            if (!(ok = mbar_wait(&wfull[s], phase, g.status))) break;
+                            umma::fence_after();
+                            const uint64_t db = db0 + (uint64_t)s * db_slot;
+#pragma unroll
+                            for (int k = 0; k < BK / 16; k++)
+                                umma::mma_bf16(d, da + 2 * k, db + 2 * k, idesc, (uint32_t)((kb | k) != 0));
+                            umma::commit(&wempty[s]);
+                            if (++s == S) {
+                                s = 0;
+                                phase ^= 1;
+                            }
+                        }
+                        if (ok) umma::commit(&dfull[t]);
+                    }
+                }
+            }
+            umma::commit(done);  // arrives once every MMA issued above has completed
+            mbar_wait(done, 0, g.status);
+        }
+    } else {
+        constexpr int NH = kEpiWarps / 4;  // epilogue warps per TMEM lane quarter
+        const int q = warp & 3, hg = (warp - 2) >> 2, ew = warp - 2;
+        const uint32_t tq = tbase + ((uint32_t)(q * 32) << 16);
+        int nd[2] = {0, 0}, nfree[2] = {0, 0};
+        // SiLU of this lane's 32 values of hidden layer l, into the activations (and kept)
+        auto finish = [&](int t, int l, long long row, int col0, const float2 (&v)[16]) {
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                uint32_t p[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const float2 y = silu2(v[4 * u + j]);
+                    p[j] = pack_bf16(y.x, y.y);
+                }
+                const uint4 pv = make_uint4(p[0], p[1], p[2], p[3]);
+                *act_unit(acts + t * AB, q * 32 + lane, col0, u) = pv;
+                if (KEEP && row < g.M) {
+                    const long long o = l * g.keep_stride + row * W + col0 + 8 * u;
+                    *reinterpret_cast<uint4 *>(g.H + o) = pv;
+                    const float2 *z = v + 4 * u;
+                    *reinterpret_cast<uint4 *>(g.Z + o) = make_uint4(pack_bf16(z[0].x, z[0].y), pack_bf16(z[1].x, z[1].y),
+                                                                     pack_bf16(z[2].x, z[2].y), pack_bf16(z[3].x, z[3].y));
+                }
+            }
+        };
+        auto ready = [&](int t) {  // this thread's part of tile t's new activations stands
+            umma::fence_before();
+            tma::fence_proxy_async();
+            umma::mbar_arrive(&act[t]);
+        };
+        auto wait_all = [&](uint64_t *bar, int n) {
+            const bool r = mbar_wait(bar, (uint32_t)(n & 1), g.status);
+            return (bool)__all_sync(0xffffffffu, r);
+        };
+        // First layer of rows base .. base + 127 into tile t.  A warp makes eight rows, a row by W / 8 lanes with
+        // eight columns each, whose weights stay in registers (a lane per row instead reads every weight in every
+        // lane: four data-path cycles per 16 bytes, 8-9k cycles per tile against the 4.1k of its SiLU).  xs: the
+        // eight rows' inputs, lane i holding values i and i + 32.
+        auto load_x = [&](long long base, float (&xs)[NIN / 4]) {
+            const long long n = (g.M - base - ew * 8) * g.n_in;  // values from the warp's first row on
+#pragma unroll
+            for (int u = 0; u < NIN / 4; u++) {
+                const int at = lane + 32 * u;
+                xs[u] = at < 8 * g.n_in && at < n ? __ldg(g.x + (base + ew * 8) * g.n_in + at) : 0.f;
+            }
+        };
+        auto first = [&](int t, long long base, const float (&xs)[NIN / 4]) {
+            const int G = W / 8, rpp = 32 / G, col0 = (lane % G) * 8;  // rows per pass
+            float2 w[NIN][4], bb[4];
+#pragma unroll
+            for (int k = 0; k < NIN; k++)
+#pragma unroll
+                for (int u = 0; u < 2; u++) {
+                    const float4 ww = k < g.n_in ? __ldg(reinterpret_cast<const float4 *>(g.W0 + k * W + col0) + u)
+                                                 : make_float4(0.f, 0.f, 0.f, 0.f);
+                    w[k][2 * u] = make_float2(ww.x, ww.y);
+                    w[k][2 * u + 1] = make_float2(ww.z, ww.w);
+                }
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                const float4 ww = __ldg(reinterpret_cast<const float4 *>(g.bias[0] + col0) + u);
+                bb[2 * u] = make_float2(ww.x, ww.y);
+                bb[2 * u + 1] = make_float2(ww.z, ww.w);
+            }
+            for (int j0 = 0; j0 < 8 && base + ew * 8 + j0 < g.M; j0 += 2 * rpp) {  // two passes at a time
+                float2 v[2][4];
+#pragma unroll
+                for (int o = 0; o < 2; o++)
+#pragma unroll
+                    for (int c = 0; c < 4; c++) v[o][c] = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int k = 0; k < NIN; k++) {
+                    if (k >= g.n_in) break;
+#pragma unroll
+                    for (int o = 0; o < 2; o++) {
+                        const int at = (j0 + o * rpp + lane / G) * g.n_in + k;
+                        float xk = __shfl_sync(0xffffffffu, xs[0], at & 31);
+                        if constexpr (NIN > 4) {
+                            const float hi = __shfl_sync(0xffffffffu, xs[1], at & 31);
+                            if (at >= 32) xk = hi;
+                        }
+#pragma unroll
+                        for (int c = 0; c < 4; c++) v[o][c] = fma2(make_float2(xk, xk), w[k][c], v[o][c]);
+                    }
+                }
+                uint32_t p[2][4];
+#pragma unroll
+                for (int o = 0; o < 2; o++)
+#pragma unroll
+                    for (int c = 0; c < 4; c++) {
+                        v[o][c] = add2(v[o][c], bb[c]);
+                        const float2 y = silu2(v[o][c]);
+                        p[o][c] = pack_bf16(y.x, y.y);
+                    }
+#pragma unroll
+                for (int o = 0; o < 2; o++) {
+                    const int r = ew * 8 + j0 + o * rpp + lane / G;
+                    const uint4 pv = make_uint4(p[o][0], p[o][1], p[o][2], p[o][3]);
+                    *act_unit(acts + t * AB, r, col0 & ~31, (col0 & 31) / 8) = pv;
+                    if (KEEP && base + r < g.M) {
+                        const long long at = (base + r) * W + col0;
+                        *reinterpret_cast<uint4 *>(g.H + at) = pv;
+                        *reinterpret_cast<uint4 *>(g.Z + at) =
+                            make_uint4(pack_bf16(v[o][0].x, v[o][0].y), pack_bf16(v[o][1].x, v[o][1].y),
+                                       pack_bf16(v[o][2].x, v[o][2].y), pack_bf16(v[o][3].x, v[o][3].y));
+                    }
+                }
+            }
+            ready(t);
+        };
+        bool ok = true;
+        // rows of this warp in tile t of group grp; a warp without rows of a tile only arrives (its accumulator
+        // rows are never read)
+        auto row_of = [&](int grp, int t) { return (long long)grp * rows_per_group + t * BM + q * 32; };
+        for (int t = 0; t < ((int)blockIdx.x < ngroups ? tiles_of(blockIdx.x) : 0); t++) {
+            float xs[NIN / 4];
+            load_x(row_of(blockIdx.x, t) - q * 32, xs);
+            first(t, row_of(blockIdx.x, t) - q * 32, xs);
+        }
+        for (int grp = blockIdx.x; ok && grp < ngroups; grp += gridDim.x) {
+            const int nt = tiles_of(grp);
+            for (int l = 1, t = 0; ok && l + 1 < nl; t + 1 < nt ? t++ : (t = 0, l++)) {  // hidden layers
+                const long long wr = row_of(grp, t);
+                if (!(ok = wait_all(&dfull[t], t ? nd[1]++ : nd[0]++))) break;
+                umma::fence_after();
+                for (int col0 = hg * 32; wr < g.M && col0 < W; col0 += 32 * NH) {
+                    float2 v[16];
+                    load_block(tq + (uint32_t)(t * kCols + col0), v);
+                    add_bias(v, g.bias[l] + col0);
+                    finish(t, l, wr + lane, col0, v);
+                }
+                ready(t);
+            }
+            // per tile: output layer, its blocks staged in the activations' place (the tile's MMAs have completed)
+            // and stored by TMA, then the first layer of the next group's tile, under the other tile's MMAs
+            const int next = grp + gridDim.x, nt_next = next < ngroups ? tiles_of(next) : 0;
+            for (int t = 0; ok && t < nt; t++) {
+                const long long wr = row_of(grp, t);
+                float xs[NIN / 4];
+                if (t < nt_next) load_x(row_of(next, t) - q * 32, xs);
+                if (!(ok = wait_all(&dfull[t], t ? nd[1]++ : nd[0]++))) break;
+                umma::fence_after();
+                unsigned char *sb = acts + t * AB + (size_t)ew * kBlockBytes;
+                for (int col0 = hg * 32; wr < g.M && col0 < g.n_out; col0 += 32 * NH) {
+                    float2 v[16];
+                    load_block(tq + (uint32_t)(t * kCols + col0), v);
+                    add_bias(v, g.bias[nl - 1] + col0);
+                    if (col0 >= 32 * NH) {  // the last block's store must have read the buffer
+                        if (lane == 0) umma::store_wait_read<0>();
+                        __syncwarp();
+                    }
+#pragma unroll
+                    for (int u = 0; u < 8; u++)  // row `lane`: 128 bytes, 16-byte unit u at u ^ (lane % 8)
+                        *reinterpret_cast<float4 *>(sb + lane * 128 + ((u ^ (lane & 7)) << 4)) =
+                            make_float4(v[2 * u].x, v[2 * u].y, v[2 * u + 1].x, v[2 * u + 1].y);
+                    tma::fence_proxy_async();
+                    __syncwarp();
+                    if (lane == 0) umma::store_2d(&mapY, col0, (int)wr, sb);
+                }
+                umma::fence_before();
+                if (t >= nt_next) continue;
+                if (lane == 0) {
+                    umma::store_wait_read<0>();
+                    umma::mbar_arrive(&sfree[t]);
+                }
+                if (!(ok = wait_all(&sfree[t], t ? nfree[1]++ : nfree[0]++))) break;
+                first(t, row_of(next, t) - q * 32, xs);
+            }
+        }
+        if (lane == 0) umma::store_wait_all();
+    }
+    umma::fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        umma::fence_after();
+        umma::tmem_free(tbase, 2 * kCols);
+    }
+}
+
+}  // namespace t6
+
 // dW = sum over splits of the partial products, db = sum of the partial
 // column sums; fixed order, so the result does not depend on scheduling.
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float *ws, const float *dbp, int splits,
@@ -796,6 +1229,9 @@ struct gabe_mlp {
     tc::WtTable wtab{};
     unsigned int *status = nullptr;  // device word: a bounded wait of the tcgen05 forward gave up
     int umma_stages[17] = {};        // per layer: ring stages of the tcgen05 forward, 0 = mma.sync kernel
+    int fused_box = 0;               // rows per weight load of it
+    int fused_slots = 0;             // weight slots of the one-launch forward (t6), 0 = layer by layer
+    CUtensorMap map_wt{};            // the stacked BF16 weights, for it
     void *Z = nullptr, *H = nullptr;  // [depth][max_rows][width] activation type
     double2 *part = nullptr;
     TrainScalars *ts = nullptr;
@@ -946,10 +1382,72 @@ int launch_umma(gabe_mlp *m, const tc::Args &a, int stages) {
     return GABE_OK;
 }
 
+// The one-launch forward takes a network whose layers after the first all run on tcgen05 and whose first
+// layer has the coalesced kernel's form; slots = weight slots that fit beside the activations (0: not taken).
+int fused_slots_for(gabe_mlp *m) {
+    const int W = m->p.width;
+    if (m->nl < 2 || m->nl > t6::kMaxLayers || m->K[0] > kFirstMaxIn || W > 256 || 256 % (W / 8) != 0) return 0;
+    for (int l = 1; l < m->nl; l++)
+        if (!m->umma_stages[l]) return 0;
+    int optin = 0;
+    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, m->dev) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    const long long s = ((long long)optin - (long long)t6::smem_bytes(W, 0)) / t6::kSlotBytes;
+    if (s < 2) return 0;
+    int rows = 0;
+    for (int l = 1; l < m->nl; l++) rows += m->N[l];
+    m->fused_box = m->p.n_out % 64 ? 32 : 64;  // divides every layer's columns
+    if (!encode_k_major(&m->map_wt, m->wt, W, rows, m->fused_box)) return 0;
+    return (int)(s > t6::kMaxSlots ? t6::kMaxSlots : s);
+}
+
+int launch_fused(gabe_mlp *m, const float *x, int rows, float *y, bool keep) {
+    CUtensorMap my;
+    if (!encode_out(&my, y, 4, m->p.n_out, rows)) return kNoTensorMap;
+    t6::Args g{};
+    g.M = rows;
+    g.width = m->p.width;
+    g.n_in = m->K[0];
+    g.n_out = m->p.n_out;
+    g.nl = m->nl;
+    g.slots = m->fused_slots;
+    g.box = m->fused_box;
+    g.x = x;
+    g.W0 = m->params + m->offW[0];
+    for (int l = 0; l < m->nl; l++) {
+        g.bias[l] = m->params + m->offb[l];
+        g.rowoff[l] = l ? (int)(m->wtab.offWt[l] / m->p.width) : 0;
+    }
+    if (keep) {
+        g.H = static_cast<bf16 *>(m->H);
+        g.Z = static_cast<bf16 *>(m->Z);
+        g.keep_stride = (long long)m->p.max_rows * m->p.width;
+    }
+    g.status = m->status;
+    int nsm = 0;
+    MCK(m, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, m->dev));
+    const int tiles = (rows + t6::BM - 1) / t6::BM;
+    g.tiles = tiles > nsm ? 2 : 1;
+    const int groups = (tiles + g.tiles - 1) / g.tiles;
+    const size_t smem = t6::smem_bytes(g.width, g.slots);
+    auto kernel = g.n_in <= 4 ? (keep ? t6::mlp_kernel<true, 4> : t6::mlp_kernel<false, 4>)
+                              : (keep ? t6::mlp_kernel<true, 8> : t6::mlp_kernel<false, 8>);
+    MCK(m, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kernel<<<groups < nsm ? groups : nsm, t6::kThreadsPerCta, smem, m->stream>>>(m->map_wt, my, g);
+    MCK(m, cudaGetLastError());
+    return GABE_OK;
+}
+
 // Input activations of layer l: x (FP32) for l = 0, H[l-1] otherwise.
 // With BF16 activations every layer after the first runs on tensor cores.
 template <typename TACT>
 int forward_rows(gabe_mlp *m, const float *x, int rows, float *y, bool keep_z) {
+    if (m->fused_slots) {
+        const int rc = launch_fused(m, x, rows, y, keep_z);
+        if (rc != kNoTensorMap) return rc;  // else: e.g. an output pointer off a 16-byte boundary
+    }
     for (int l = 0; l < m->nl; l++) {
         if (l == 0 && m->nl > 1 && m->K[0] <= kFirstMaxIn && 256 % (m->N[0] / 8) == 0) {
             launch_first_n<TACT>(m->K[0], x, rows, m->params + m->offW[0], m->params + m->offb[0], m->N[0],
@@ -1217,6 +1715,7 @@ int gabe_mlp_create(const gabe_mlp_params *p, gabe_mlp **out) {
     if (!m->f32act && !(p->flags & GABE_MLP_MMA_SYNC))
         for (int l = 1; l < m->nl; l++)
             m->umma_stages[l] = umma_stages_for(m->dev, m->K[l], m->N[l], l + 1 == m->nl ? 4 : 2);
+    m->fused_slots = fused_slots_for(m);
     *out = m;
     return GABE_OK;
 }
@@ -1372,11 +1871,13 @@ int gabe_mlp_forward_form(const gabe_mlp *m, int32_t layer) {
 void *gabe_mlp_stream(const gabe_mlp *m) { return m ? (void *)m->stream : nullptr; }
 
 int gabe_mlp_launches_per_train_step(const gabe_mlp *m) {
-    return m ? 3 + 3 * m->nl + (m->nl - 1) + (m->f32act ? 0 : 1) : 0;
+    return m ? 3 + (m->fused_slots ? 1 : m->nl) + 2 * m->nl + (m->nl - 1) + (m->f32act ? 0 : 1) : 0;
 }
 
 
-int gabe_mlp_launches_per_forward(const gabe_mlp *m) { return m ? m->nl : 0; }
+int gabe_mlp_launches_per_forward(const gabe_mlp *m) {
+    return m ? (m->fused_slots ? 1 : m->nl) : 0;
+}
 
 const char *gabe_mlp_last_error(const gabe_mlp *m) { return m ? m->err.c_str() : g_mlp_create_error.c_str(); }
 

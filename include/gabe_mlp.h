@@ -12,7 +12,9 @@
  * weights fit in shared memory (K <= 256, N <= 256, K a multiple of 64, N
  * of 32) runs on the fifth-generation tensor cores (tcgen05, TMEM
  * accumulators), other BF16 layers on mma.sync, the first layer and the
- * backward products on FP32 FMA.  Flat parameter layout, layer by layer:
+ * backward products on FP32 FMA.  Where every layer after the first has that
+ * form (width 64, 128 or 256, at most 8 inputs) the forward is one launch
+ * that keeps the activations on chip.  Flat parameter layout, layer by layer:
  * W_l [K_l][N_l] (row-major, K_l inputs) followed by b_l [N_l].
  *
  * Targets may hold NaN (log bins with no native bin): the loss is the mean

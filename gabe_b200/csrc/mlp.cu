@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <cstdint>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -95,17 +96,18 @@ struct GemmArgs {
 constexpr int BM = 64, BN = 64, BK = 16, kThreads = 256;
 
 // TA: type of A; TACT: activation storage type (Z/H of the epilogues).
+// Tile (bx, by) of the output, split bz of k (EPI_BWD_WEIGHT).
 template <typename TA, typename TACT, int EPI>
-__global__ void __launch_bounds__(kThreads) gemm_kernel(GemmArgs g) {
+__device__ __forceinline__ void gemm_tile(const GemmArgs &g, int bx, int by, int bz) {
     __shared__ __align__(16) float As[BK][BM];
     __shared__ __align__(16) float Bs[BK][BN];
     const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    const int m0 = by * BM, n0 = bx * BN;
     const TA *A = static_cast<const TA *>(g.A);
     float acc[4][4] = {};
     // split-K (weight gradient): this block sums k in [kb, ke) and writes
-    // its partial product to slice blockIdx.z of the output
-    const int kb = EPI == EPI_BWD_WEIGHT ? blockIdx.z * g.kchunk : 0;
+    // its partial product to slice bz of the output
+    const int kb = EPI == EPI_BWD_WEIGHT ? bz * g.kchunk : 0;
     const int ke = EPI == EPI_BWD_WEIGHT ? min(g.K, kb + g.kchunk) : g.K;
     float csum = 0.f;  // EPI_BWD_WEIGHT, first row of tiles: column sums of B (the bias gradient)
     for (int k0 = kb; k0 < ke; k0 += BK) {
@@ -143,7 +145,7 @@ __global__ void __launch_bounds__(kThreads) gemm_kernel(GemmArgs g) {
             }
         }
         __syncthreads();
-        if (EPI == EPI_BWD_WEIGHT && blockIdx.y == 0 && tid < BN) {
+        if (EPI == EPI_BWD_WEIGHT && by == 0 && tid < BN) {
 #pragma unroll
             for (int kk = 0; kk < BK; kk++) csum += Bs[kk][tid];
         }
@@ -159,9 +161,9 @@ __global__ void __launch_bounds__(kThreads) gemm_kernel(GemmArgs g) {
         }
         __syncthreads();
     }
-    if (EPI == EPI_BWD_WEIGHT && blockIdx.y == 0 && tid < BN && n0 + tid < g.N)
-        g.dbp[(long long)blockIdx.z * g.N + n0 + tid] = csum;
-    float *Cz = static_cast<float *>(g.C) + (EPI == EPI_BWD_WEIGHT ? (long long)blockIdx.z * g.M * g.ldc : 0);
+    if (EPI == EPI_BWD_WEIGHT && by == 0 && tid < BN && n0 + tid < g.N)
+        g.dbp[(long long)bz * g.N + n0 + tid] = csum;
+    float *Cz = static_cast<float *>(g.C) + (EPI == EPI_BWD_WEIGHT ? (long long)bz * g.M * g.ldc : 0);
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const int m = m0 + ty * 4 + i;
@@ -185,6 +187,104 @@ __global__ void __launch_bounds__(kThreads) gemm_kernel(GemmArgs g) {
             }
         }
     }
+}
+
+template <typename TA, typename TACT, int EPI>
+__global__ void __launch_bounds__(kThreads) gemm_kernel(GemmArgs g) {
+    gemm_tile<TA, TACT, EPI>(g, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+
+// Weight gradients of every layer in one launch (batches of at most
+// kSmallRows): block b takes tile and split b - first[l] of layer l.
+constexpr int kMaxGradLayers = 17;
+struct WeightGradArgs {
+    int nl, first[kMaxGradLayers + 1];
+    GemmArgs g[kMaxGradLayers];
+};
+template <typename TACT>
+__global__ void __launch_bounds__(kThreads) weight_grad_kernel(const __grid_constant__ WeightGradArgs a) {
+    int l = 0;
+    while (l + 1 < a.nl && (int)blockIdx.x >= a.first[l + 1]) l++;
+    const GemmArgs &g = a.g[l];
+    const int b = blockIdx.x - a.first[l], nx = (g.N + BN - 1) / BN, ny = (g.M + BM - 1) / BM;
+    const int bx = b % nx, by = (b / nx) % ny, bz = b / (nx * ny);
+    if (l == 0) gemm_tile<float, TACT, EPI_BWD_WEIGHT>(g, bx, by, bz);
+    else gemm_tile<TACT, TACT, EPI_BWD_WEIGHT>(g, bx, by, bz);
+}
+
+// Data gradient of a small batch: C[m][n] = (sum_k A[m][k] W[n][k])
+// SiLU'(Z[m][n]), both operands contiguous along k.  32 x 32 outputs per
+// block (four per thread), so that a 512 x 256 product makes 128 blocks
+// instead of the tiled kernel's 32 of 64 x 64, whose 16 latency-bound k slices
+// took 28 us; here the operands of 128 k at a time land by cp.async, one slice
+// ahead.  Every output sums its k in order on one FP32 accumulator, as the
+// tiled kernel does: the same bits.  Needs K % 4 == 0.
+constexpr int kDgT = 256, kDgTile = 32, kDgK = 128, kDgPitch = kDgK + 4;
+constexpr size_t kDgSmem = (size_t)2 * 2 * kDgTile * kDgPitch * sizeof(float);
+template <typename TACT>
+__global__ void __launch_bounds__(kDgT) data_grad_kernel(const float *A, const float *W, const TACT *Z, float *C, int M,
+                                                         int N, int K) {
+    extern __shared__ __align__(16) float dg[];  // [2 stages][A, W][32][pitch]
+    const int tid = threadIdx.x, m0 = blockIdx.y * kDgTile, n0 = blockIdx.x * kDgTile;
+    auto stage = [&](int st, int op) { return dg + (st * 2 + op) * kDgTile * kDgPitch; };
+    auto load = [&](int st, int k0) {
+        for (int t = tid; t < 2 * kDgTile * (kDgK / 4); t += kDgT) {
+            const int op = t / (kDgTile * (kDgK / 4)), r = (t / (kDgK / 4)) % kDgTile, c = 4 * (t % (kDgK / 4));
+            const int row = (op ? n0 : m0) + r, k = k0 + c;
+            float *dst = stage(st, op) + r * kDgPitch + c;
+            if (row < (op ? N : M) && k < K) {
+                const float *src = (op ? W : A) + (long long)row * K + k;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                             "l"(src)
+                             : "memory");
+            } else {
+                *reinterpret_cast<float4 *>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    const int tx = tid % 16, ty = tid / 16;  // rows ty, ty + 16; columns tx, tx + 16
+    float acc[2][2] = {};
+    load(0, 0);
+    for (int k0 = 0, st = 0; k0 < K; k0 += kDgK, st ^= 1) {
+        if (k0 + kDgK < K) {
+            load(st ^ 1, k0 + kDgK);
+            asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        }
+        __syncthreads();
+        const float *a = stage(st, 0) + ty * kDgPitch, *w = stage(st, 1) + tx * kDgPitch;
+        const int kn = min(kDgK, K - k0);
+#pragma unroll 8
+        for (int k = 0; k < kn; k += 4) {
+            float4 av[2], wv[2];
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                av[i] = *reinterpret_cast<const float4 *>(a + i * 16 * kDgPitch + k);
+                wv[i] = *reinterpret_cast<const float4 *>(w + i * 16 * kDgPitch + k);
+            }
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+#pragma unroll
+                for (int j = 0; j < 2; j++) {
+                    acc[i][j] = fmaf(av[i].x, wv[j].x, acc[i][j]);
+                    acc[i][j] = fmaf(av[i].y, wv[j].y, acc[i][j]);
+                    acc[i][j] = fmaf(av[i].z, wv[j].z, acc[i][j]);
+                    acc[i][j] = fmaf(av[i].w, wv[j].w, acc[i][j]);
+                }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const int m = m0 + ty + 16 * i, n = n0 + tx + 16 * j;
+            if (m >= M || n >= N) continue;
+            const long long o = (long long)m * N + n;
+            C[o] = acc[i][j] * dsilu(ldf(Z, o));
+        }
 }
 
 // Forward of the first layer (NIN <= 8 inputs): z = x W0 + b0, h = SiLU(z),
@@ -391,14 +491,21 @@ __global__ void __launch_bounds__(T, 2) gemm_tc_kernel(Args g) {
             for (int nf = 0; nf < 4; nf++) {
                 const int n = n0 + wn * 32 + nf * 8 + gc;
                 if (n >= g.N) continue;
-                const float z0 = acc[mf][nf][2 * h] + g.bias[n], z1 = acc[mf][nf][2 * h + 1] + g.bias[n + 1];
+                const bool pair = n + 1 < g.N;  // an odd number of outputs ends in a single column
+                const float z0 = acc[mf][nf][2 * h] + g.bias[n], z1 = acc[mf][nf][2 * h + 1] + (pair ? g.bias[n + 1] : 0.f);
                 const long long o = (long long)m * g.N + n;
                 if constexpr (EPI == EPI_HIDDEN) {
                     if (g.Z) *reinterpret_cast<__nv_bfloat162 *>(g.Z + o) = __floats2bfloat162_rn(z0, z1);
                     *reinterpret_cast<__nv_bfloat162 *>(static_cast<bf16 *>(g.C) + o) =
                         __floats2bfloat162_rn(silu(z0), silu(z1));
                 } else {
-                    *reinterpret_cast<float2 *>(static_cast<float *>(g.C) + o) = make_float2(z0, z1);
+                    float *c = static_cast<float *>(g.C) + o;
+                    if (pair && (reinterpret_cast<uintptr_t>(c) & 7) == 0) {
+                        *reinterpret_cast<float2 *>(c) = make_float2(z0, z1);
+                    } else {
+                        c[0] = z0;
+                        if (pair) c[1] = z1;
+                    }
                 }
             }
         }
@@ -775,6 +882,12 @@ __device__ __forceinline__ void add_bias(float2 (&v)[16], const float *b) {
         v[2 * u + 1] = add2(v[2 * u + 1], make_float2(bb.z, bb.w));
     }
 }
+// 32 bytes in one store (32-byte aligned): half the line touches of two 16-byte ones where each lane writes a row.
+__device__ __forceinline__ void store32(void *p, const uint4 &a, const uint4 &b) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w),
+                 "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
+                 : "memory");
+}
 // This lane's row of 32 accumulator columns.
 __device__ __forceinline__ void load_block(uint32_t taddr, float2 (&v)[16]) {
     float f[32];
@@ -904,21 +1017,27 @@ __global__ void __launch_bounds__(kThreadsPerCta, 1)
         // SiLU of this lane's 32 values of hidden layer l, into the activations (and kept)
         auto finish = [&](int t, int l, long long row, int col0, const float2 (&v)[16]) {
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
-                uint32_t p[4];
+            for (int u = 0; u < 4; u += 2) {
+                uint4 pv[2], zv[2];
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const float2 y = silu2(v[4 * u + j]);
-                    p[j] = pack_bf16(y.x, y.y);
+                for (int o = 0; o < 2; o++) {
+                    uint32_t p[4];
+                    const float2 *z = v + 4 * (u + o);
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        const float2 y = silu2(z[j]);
+                        p[j] = pack_bf16(y.x, y.y);
+                    }
+                    pv[o] = make_uint4(p[0], p[1], p[2], p[3]);
+                    if (KEEP)
+                        zv[o] = make_uint4(pack_bf16(z[0].x, z[0].y), pack_bf16(z[1].x, z[1].y),
+                                           pack_bf16(z[2].x, z[2].y), pack_bf16(z[3].x, z[3].y));
+                    *act_unit(acts + t * AB, q * 32 + lane, col0, u + o) = pv[o];
                 }
-                const uint4 pv = make_uint4(p[0], p[1], p[2], p[3]);
-                *act_unit(acts + t * AB, q * 32 + lane, col0, u) = pv;
                 if (KEEP && row < g.M) {
                     const long long o = l * g.keep_stride + row * W + col0 + 8 * u;
-                    *reinterpret_cast<uint4 *>(g.H + o) = pv;
-                    const float2 *z = v + 4 * u;
-                    *reinterpret_cast<uint4 *>(g.Z + o) = make_uint4(pack_bf16(z[0].x, z[0].y), pack_bf16(z[1].x, z[1].y),
-                                                                     pack_bf16(z[2].x, z[2].y), pack_bf16(z[3].x, z[3].y));
+                    store32(g.H + o, pv[0], pv[1]);
+                    store32(g.Z + o, zv[0], zv[1]);
                 }
             }
         };
@@ -1154,13 +1273,21 @@ __global__ void __launch_bounds__(256) loss_kernel(const float *y, const float *
         last = atomicAdd(&ts->counter, 1u) == gridDim.x - 1;
     }
     __syncthreads();
-    if (last && threadIdx.x == 0) {
-        __threadfence();
+    if (!last) return;
+    // the block partials arrive together, and are added in block order
+    __threadfence();
+    static_assert(kLossBlocks <= 256, "one partial per thread");
+    if (threadIdx.x < gridDim.x) {
+        const double2 p = __ldcg(&part[threadIdx.x]);
+        rs[threadIdx.x] = p.x;
+        rc[threadIdx.x] = p.y;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
         double S = 0., C = 0.;
         for (unsigned b = 0; b < gridDim.x; b++) {
-            const double2 p = __ldcg(&part[b]);
-            S += p.x;
-            C += p.y;
+            S += rs[b];
+            C += rc[b];
         }
         const double L = C > 0. ? S / C : 0.;
         ts->loss_last = L;
@@ -1187,27 +1314,118 @@ struct AdamHyper {
     long long decay_steps;  // cosine from lr to lr_min over this many steps (0 = constant lr)
 };
 
-// AdamW with bias correction; the gradient is the unnormalised batch
-// gradient times 1/count.
+// The step's scalars: 1/count, bias corrections, learning rate.
+struct AdamStep {
+    float inv, bc1, bc2, lr;
+};
+__device__ __forceinline__ float adam_correction(float beta, const TrainScalars *ts) {
+    return (float)(1. - pow((double)beta, (double)ts->step));
+}
+__device__ __forceinline__ float adam_rate(const AdamHyper &h, const TrainScalars *ts) {
+    if (h.decay_steps <= 0) return h.lr;
+    const double t = (double)ts->step, f = fmin(t - 1., (double)h.decay_steps) / (double)h.decay_steps;
+    return (float)(h.lr_min + 0.5 * (h.lr - h.lr_min) * (1. + cos(M_PI * f)));
+}
+__device__ __forceinline__ AdamStep adam_step(const AdamHyper &h, const TrainScalars *ts) {
+    return AdamStep{ts->inv_count, adam_correction(h.b1, ts), adam_correction(h.b2, ts), adam_rate(h, ts)};
+}
+
+// AdamW with bias correction of parameter i; g is the unnormalised batch
+// gradient.  Returns the new value.
+__device__ __forceinline__ float adam_update(float *p, float *m, float *v, long long i, float g, const AdamHyper &h,
+                                             const AdamStep &a) {
+    // the roundings are spelled out, so that every kernel that takes this step gives the same bits
+    const float gi = __fmul_rn(g, a.inv);
+    float pi = p[i];
+    pi = __fmaf_rn(-__fmul_rn(a.lr, h.wd), pi, pi);
+    const float mi = __fmaf_rn(1.f - h.b1, gi, __fmul_rn(h.b1, m[i]));
+    const float vi = __fmaf_rn(__fmul_rn(1.f - h.b2, gi), gi, __fmul_rn(h.b2, v[i]));
+    m[i] = mi;
+    v[i] = vi;
+    return p[i] = __fsub_rn(pi, __fdiv_rn(__fmul_rn(a.lr, __fdiv_rn(mi, a.bc1)),
+                                          __fadd_rn(__fsqrt_rn(__fdiv_rn(vi, a.bc2)), h.eps)));
+}
+
 __global__ void adam_kernel(float *p, const float *g, float *m, float *v, long long n, AdamHyper h,
                             const TrainScalars *ts) {
-    const float inv = ts->inv_count;
-    const double t = (double)ts->step;
-    const float bc1 = (float)(1. - pow((double)h.b1, t)), bc2 = (float)(1. - pow((double)h.b2, t));
-    float lr = h.lr;
-    if (h.decay_steps > 0) {
-        const double f = fmin(t - 1., (double)h.decay_steps) / (double)h.decay_steps;
-        lr = (float)(h.lr_min + 0.5 * (h.lr - h.lr_min) * (1. + cos(M_PI * f)));
+    const AdamStep a = adam_step(h, ts);
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+        adam_update(p, m, v, i, g[i], h, a);
+}
+
+// End of a small batch's step in one launch: adds the split-K partials of
+// every gradient in order, takes the AdamW step and writes the BF16
+// transposed copy of the new weight (GRAD: stores the normalised gradient
+// instead).  A block takes a 32 x 32 tile of one layer's weights, transposed
+// through shared memory, or 256 biases.
+struct UpdateArgs {
+    int nl, first[kMaxGradLayers + 1];  // first block of layer l: its weight tiles, then its biases
+    int K[kMaxGradLayers], N[kMaxGradLayers], splits[kMaxGradLayers];
+    long long offW[kMaxGradLayers], offb[kMaxGradLayers], offWt[kMaxGradLayers];
+    const float *ws[kMaxGradLayers], *dbp[kMaxGradLayers];
+    float *p, *m, *v, *grads;
+    bf16 *wt;  // null: no BF16 copy
+    AdamHyper h;
+    const TrainScalars *ts;
+};
+__device__ __forceinline__ float sum_splits(const float *ws, long long stride, int splits) {
+    float s = 0.f;
+    for (int z0 = 0; z0 < splits; z0 += 8) {  // eight loads in flight, added in order
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) v[u] = z0 + u < splits ? ws[(z0 + u) * stride] : 0.f;
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            if (z0 + u < splits) s += v[u];
     }
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const float gi = g[i] * inv;
-        float pi = p[i];
-        pi -= lr * h.wd * pi;
-        const float mi = h.b1 * m[i] + (1.f - h.b1) * gi;
-        const float vi = h.b2 * v[i] + (1.f - h.b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        p[i] = pi - lr * (mi / bc1) / (sqrtf(vi / bc2) + h.eps);
+    return s;
+}
+template <bool GRAD>
+__global__ void __launch_bounds__(256) update_kernel(const __grid_constant__ UpdateArgs a) {
+    __shared__ AdamStep step;
+    __shared__ bf16 tile[32][33];
+    // the scalars by one warp each (FP64 powers), while the gradients are summed
+    if (threadIdx.x == 0) step.inv = a.ts->inv_count;
+    if (!GRAD && threadIdx.x == 32) step.bc1 = adam_correction(a.h.b1, a.ts);
+    if (!GRAD && threadIdx.x == 64) step.bc2 = adam_correction(a.h.b2, a.ts);
+    if (!GRAD && threadIdx.x == 96) step.lr = adam_rate(a.h, a.ts);
+    int l = 0;
+    while (l + 1 < a.nl && (int)blockIdx.x >= a.first[l + 1]) l++;
+    const int b = blockIdx.x - a.first[l], K = a.K[l], N = a.N[l];
+    const int nx = (N + 31) / 32, tiles = nx * ((K + 31) / 32);
+    auto put = [&](long long i, float g) {
+        if constexpr (GRAD) return a.grads[i] = g * step.inv;
+        else return adam_update(a.p, a.m, a.v, i, g, a.h, step);
+    };
+    if (b >= tiles) {
+        const int n = (b - tiles) * 256 + threadIdx.x;
+        const float g = n < N ? sum_splits(a.dbp[l] + n, N, a.splits[l]) : 0.f;
+        __syncthreads();
+        if (n < N) put(a.offb[l] + n, g);
+        return;
+    }
+    const int k0 = (b / nx) * 32, n0 = (b % nx) * 32, x = threadIdx.x % 32, y = threadIdx.x / 32;
+    float g[4];
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+        const int k = k0 + y + 8 * r, n = n0 + x;
+        g[r] = k < K && n < N ? sum_splits(a.ws[l] + (long long)k * N + n, (long long)K * N, a.splits[l]) : 0.f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+        const int k = k0 + y + 8 * r, n = n0 + x;
+        if (k < K && n < N) {
+            const float w = put(a.offW[l] + (long long)k * N + n, g[r]);
+            if (!GRAD) tile[x][y + 8 * r] = __float2bfloat16_rn(w);
+        }
+    }
+    if (GRAD || !a.wt || l == 0) return;
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < 32; r += 8) {
+        const int n = n0 + y + r, k = k0 + x;
+        if (k < K && n < N) a.wt[a.offWt[l] + (long long)n * K + k] = tile[y + r][x];
     }
 }
 
@@ -1225,6 +1443,10 @@ struct gabe_mlp {
     float *params = nullptr, *grads = nullptr, *mom = nullptr, *vel = nullptr;
     float *xb = nullptr, *tb = nullptr, *y = nullptr, *dy = nullptr, *d0 = nullptr, *d1 = nullptr;
     float *ws = nullptr, *dbp = nullptr;  // split-K partials of the weight gradient
+    // batches of at most kSmallRows rows: every layer's gradient of the pre-activations and split-K partials
+    float *small_delta = nullptr, *small_ws = nullptr;
+    int small_rows = 0;
+    std::vector<long long> small_off;  // floats: per layer, weight partials then bias partials
     bf16 *wt = nullptr;              // BF16 transposed weights of layers >= 1 (tensor-core forward)
     tc::WtTable wtab{};
     unsigned int *status = nullptr;  // device word: a bounded wait of the tcgen05 forward gave up
@@ -1270,6 +1492,23 @@ void *act_at(const gabe_mlp *m, void *base, int layer) {
 }
 
 constexpr int kMaxSplits = 16;
+// Batches up to here take the one-launch weight gradients and update, which keep every layer's deltas and
+// partials at once (a bounded buffer); larger ones are long enough per launch.
+constexpr int kSmallRows = 4096;
+
+// Splits of the batch for the weight gradient of a K x N layer, enough for about two blocks per SM, and the
+// rows of one split.
+int most_splits(int K, int N) {
+    const int tiles = ((K + BM - 1) / BM) * ((N + BN - 1) / BN), splits = (296 + tiles - 1) / tiles;
+    return splits < 1 ? 1 : (splits > kMaxSplits ? kMaxSplits : splits);
+}
+int weight_grad_splits(int K, int N, int rows, int *chunk) {
+    const int splits = most_splits(K, N);
+    int c = (rows + splits - 1) / splits;
+    c = (c + BK - 1) / BK * BK;
+    *chunk = c;
+    return (rows + c - 1) / c;
+}
 
 template <typename TA, typename TACT, int EPI>
 int launch_gemm(gabe_mlp *m, const GemmArgs &g, int splits = 1) {
@@ -1523,14 +1762,7 @@ int backward_rows(gabe_mlp *m, const float *x, int rows) {
         w.C = m->ws;
         w.ldc = N;
         w.dbp = m->dbp;
-        // enough splits of the batch to give about two blocks per SM
-        const int tiles = ((K + BM - 1) / BM) * ((N + BN - 1) / BN);
-        int splits = (296 + tiles - 1) / tiles;
-        splits = splits < 1 ? 1 : (splits > kMaxSplits ? kMaxSplits : splits);
-        int chunk = (rows + splits - 1) / splits;
-        chunk = (chunk + BK - 1) / BK * BK;
-        splits = (rows + chunk - 1) / chunk;
-        w.kchunk = chunk;
+        const int splits = weight_grad_splits(K, N, rows, &w.kchunk);
         int rc = l == 0 ? launch_gemm<float, TACT, EPI_BWD_WEIGHT>(m, w, splits)
                         : launch_gemm<TACT, TACT, EPI_BWD_WEIGHT>(m, w, splits);
         if (rc) return rc;
@@ -1559,6 +1791,92 @@ int backward_rows(gabe_mlp *m, const float *x, int rows) {
     return GABE_OK;
 }
 
+// A small batch's backward: the data gradients layer by layer, then every weight gradient in one launch, then
+// (step) the AdamW step and the BF16 weights, or (!step) the normalised gradients, in another.
+template <typename TACT>
+int backward_small(gabe_mlp *m, const float *x, int rows, bool step) {
+    const int nl = m->nl;
+    std::vector<const float *> delta(nl);
+    delta[nl - 1] = m->dy;
+    for (int l = nl - 1; l > 0; l--) {
+        const int K = m->K[l], N = m->N[l];
+        float *out = m->small_delta + (size_t)(l - 1) * m->small_rows * m->p.width;
+        if (N % 4 == 0) {
+            const dim3 grid((K + kDgTile - 1) / kDgTile, (rows + kDgTile - 1) / kDgTile);
+            MCK(m, cudaFuncSetAttribute(data_grad_kernel<TACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgSmem));
+            data_grad_kernel<TACT><<<grid, kDgT, kDgSmem, m->stream>>>(
+                delta[l], m->params + m->offW[l], static_cast<const TACT *>(act_at(m, m->Z, l - 1)), out, rows, K, N);
+            MCK(m, cudaGetLastError());
+        } else {
+            GemmArgs d{};
+            d.M = rows;
+            d.N = K;
+            d.K = N;
+            d.A = delta[l];
+            d.sam = N;
+            d.sak = 1;
+            d.B = m->params + m->offW[l];
+            d.sbk = 1;
+            d.sbn = N;
+            d.Z = act_at(m, m->Z, l - 1);
+            d.C = out;
+            d.ldc = K;
+            const int rc = launch_gemm<float, TACT, EPI_BWD_DATA>(m, d);
+            if (rc) return rc;
+        }
+        delta[l - 1] = out;
+    }
+    WeightGradArgs w{};
+    UpdateArgs u{};
+    w.nl = u.nl = nl;
+    int wb = 0, ub = 0;
+    for (int l = 0; l < nl; l++) {
+        const int K = m->K[l], N = m->N[l];
+        GemmArgs &g = w.g[l];
+        g.M = K;
+        g.N = N;
+        g.K = rows;
+        g.A = l == 0 ? static_cast<const void *>(x) : act_at(m, m->H, l - 1);
+        g.sam = 1;
+        g.sak = K;
+        g.B = delta[l];
+        g.sbk = N;
+        g.sbn = 1;
+        u.splits[l] = weight_grad_splits(K, N, rows, &g.kchunk);
+        g.C = m->small_ws + m->small_off[2 * l];
+        g.ldc = N;
+        g.dbp = m->small_ws + m->small_off[2 * l + 1];
+        w.first[l] = wb;
+        wb += ((K + BM - 1) / BM) * ((N + BN - 1) / BN) * u.splits[l];
+        u.K[l] = K;
+        u.N[l] = N;
+        u.offW[l] = m->offW[l];
+        u.offb[l] = m->offb[l];
+        u.offWt[l] = m->wtab.offWt[l];
+        u.ws[l] = static_cast<const float *>(g.C);
+        u.dbp[l] = g.dbp;
+        u.first[l] = ub;
+        ub += ((K + 31) / 32) * ((N + 31) / 32) + (N + 255) / 256;
+    }
+    weight_grad_kernel<TACT><<<wb, kThreads, 0, m->stream>>>(w);
+    MCK(m, cudaGetLastError());
+    u.p = m->params;
+    u.m = m->mom;
+    u.v = m->vel;
+    u.grads = m->grads;
+    u.wt = m->f32act ? nullptr : m->wt;
+    u.h = AdamHyper{m->p.lr, m->p.beta1, m->p.beta2, m->p.eps, m->p.weight_decay, m->p.lr_min, m->p.decay_steps};
+    u.ts = m->ts;
+    if (step) update_kernel<false><<<ub, 256, 0, m->stream>>>(u);
+    else update_kernel<true><<<ub, 256, 0, m->stream>>>(u);
+    MCK(m, cudaGetLastError());
+    return GABE_OK;
+}
+
+int bwd_small(gabe_mlp *m, const float *x, int rows, bool step) {
+    return m->f32act ? backward_small<float>(m, x, rows, step) : backward_small<bf16>(m, x, rows, step);
+}
+
 int fwd(gabe_mlp *m, const float *x, int rows, float *y, bool keep_z) {
     return m->f32act ? forward_rows<float>(m, x, rows, y, keep_z) : forward_rows<bf16>(m, x, rows, y, keep_z);
 }
@@ -1575,6 +1893,7 @@ int train_step(gabe_mlp *m, const float *x, const float *t, const int32_t *perm,
     if (rc) return rc;
     loss_kernel<<<kLossBlocks, 256, 0, m->stream>>>(m->y, m->tb, (long long)B * nout, m->dy, m->part, m->ts, 1);
     MCK(m, cudaGetLastError());
+    if (B <= m->small_rows) return bwd_small(m, m->xb, B, true);
     if ((rc = bwd(m, m->xb, B))) return rc;
     AdamHyper h{m->p.lr, m->p.beta1, m->p.beta2, m->p.eps, m->p.weight_decay, m->p.lr_min, m->p.decay_steps};
     adam_kernel<<<148 * 4, 256, 0, m->stream>>>(m->params, m->grads, m->mom, m->vel, m->P, h, m->ts);
@@ -1593,7 +1912,7 @@ void free_all(gabe_mlp *m) {
     if (m->gexec) cudaGraphExecDestroy(m->gexec);
     if (m->graph) cudaGraphDestroy(m->graph);
     void *bufs[] = {m->params, m->grads, m->mom, m->vel, m->xb, m->tb, m->y, m->dy, m->d0, m->d1, m->Z, m->H,
-                    m->part, m->ts, m->ws, m->dbp, m->wt, m->status};
+                    m->part, m->ts, m->ws, m->dbp, m->wt, m->status, m->small_delta, m->small_ws};
     for (void *b : bufs)
         if (b) cudaFree(b);
     if (m->stream) cudaStreamDestroy(m->stream);
@@ -1671,6 +1990,15 @@ int gabe_mlp_create(const gabe_mlp_params *p, gabe_mlp **out) {
     }
     const size_t R = p->max_rows, W = p->width, A = act_size(m);
     const size_t wide = (size_t)(p->n_out > p->width ? p->n_out : p->width);
+    m->small_rows = p->max_rows < kSmallRows ? p->max_rows : kSmallRows;
+    long long small_ws = 0;
+    for (int l = 0; l < m->nl; l++) {
+        const long long splits = most_splits(m->K[l], m->N[l]);
+        m->small_off.push_back(small_ws);
+        small_ws += splits * m->K[l] * m->N[l];
+        m->small_off.push_back(small_ws);
+        small_ws += splits * m->N[l];
+    }
     struct {
         void **ptr;
         size_t bytes;
@@ -1682,6 +2010,7 @@ int gabe_mlp_create(const gabe_mlp_params *p, gabe_mlp **out) {
         {(void **)&m->part, kLossBlocks * sizeof(double2)}, {(void **)&m->ts, sizeof(TrainScalars)},
         {(void **)&m->ws, (size_t)kMaxSplits * wide * wide * 4}, {(void **)&m->dbp, (size_t)kMaxSplits * wide * 4},
         {(void **)&m->wt, (size_t)(nwt > 0 ? nwt : 1) * sizeof(bf16)}, {(void **)&m->status, sizeof(unsigned int)},
+        {(void **)&m->small_delta, (size_t)p->depth * m->small_rows * W * 4}, {(void **)&m->small_ws, (size_t)small_ws * 4},
     };
     for (auto &a : allocs) {
         if (cudaMalloc(a.ptr, a.bytes) != cudaSuccess) {
@@ -1769,9 +2098,13 @@ int gabe_mlp_loss_grad(gabe_mlp *m, const float *x, const float *t, int64_t n, d
     loss_kernel<<<kLossBlocks, 256, 0, m->stream>>>(m->y, t, (long long)rows * m->p.n_out, m->dy, m->part, m->ts, 0);
     MCK(m, cudaGetLastError());
     if (h_grad) {
-        if ((rc = bwd(m, x, rows))) return rc;
-        scale_kernel<<<148, 256, 0, m->stream>>>(m->grads, m->P, m->ts);
-        MCK(m, cudaGetLastError());
+        if (rows <= m->small_rows) {
+            if ((rc = bwd_small(m, x, rows, false))) return rc;
+        } else {
+            if ((rc = bwd(m, x, rows))) return rc;
+            scale_kernel<<<148, 256, 0, m->stream>>>(m->grads, m->P, m->ts);
+            MCK(m, cudaGetLastError());
+        }
         MCK(m, cudaMemcpyAsync(h_grad, m->grads, m->P * 4, cudaMemcpyDeviceToHost, m->stream));
     }
     TrainScalars ts;
@@ -1871,7 +2204,8 @@ int gabe_mlp_forward_form(const gabe_mlp *m, int32_t layer) {
 void *gabe_mlp_stream(const gabe_mlp *m) { return m ? (void *)m->stream : nullptr; }
 
 int gabe_mlp_launches_per_train_step(const gabe_mlp *m) {
-    return m ? 3 + (m->fused_slots ? 1 : m->nl) + 2 * m->nl + (m->nl - 1) + (m->f32act ? 0 : 1) : 0;
+    // batches of at most kSmallRows: gather, forward, loss, data gradients, weight gradients, update
+    return m ? 2 + (m->fused_slots ? 1 : m->nl) + (m->nl - 1) + 2 : 0;
 }
 
 

@@ -60,6 +60,9 @@ struct StencilArgs {
     // instead of finishing the stage; the caller adds the totals of all
     // slabs and finishes with slab_finish_kernel.
     double *sums_out;
+    // Host memory (mapped) that receives the scalars after the last block has
+    // finished the stage, or null: a caller that waits for them saves the copy.
+    DevScalars *mirror;
 };
 
 constexpr int kNV = 8;  // reduced values: kin0 pot0 grad0 | pot1 grad1 PP PQ QQ
@@ -531,6 +534,7 @@ __global__ void __launch_bounds__(TK *TJ) sweep_kernel(StencilArgs args) {
                 for (int q = 0; q < kNV; q++) args.sums_out[q] = tot[q];
             else
                 finish_a<T, MODE>(c, args.sc, tot, args.slot);
+            if (args.mirror) *args.mirror = *args.sc;
             *args.counter = 0u;
         }
     } else if (tid == 0) {

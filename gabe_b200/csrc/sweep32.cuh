@@ -373,6 +373,7 @@ __global__ void __launch_bounds__(TK2 *TJ, (sweep32_threads_per_sm<MODE>() + TK2
                 for (int q = 0; q < kNV; q++) args.sums_out[q] = tot[q];
             else
                 finish_a<float, MODE>(c, args.sc, tot, args.slot);
+            if (args.mirror) *args.mirror = *args.sc;
             *args.counter = 0u;
         }
     } else if (tid == 0) {

@@ -84,33 +84,88 @@ __device__ __forceinline__ double dv64(const LatticeConsts &c, int fld, double P
 // V'(fbar+d) - V'(fbar) expanded so that no term cancels (pb, cb = homogeneous
 // phi, chi; a, b = their fluctuations).
 // ---------------------------------------------------------------------------
-struct MeanF {
-    float pb, cb;      // homogeneous values as float
-    float q0, q1;      // model constants as float
-    float q2, q3;
-    float pb2, cb2;    // 2 pb, 2 cb
-    float pbsq, pb3sq; // pb^2, 3 pb^2
+// Two FP32 values in one register pair, worked on by the packed FP32 units of
+// sm_100 (one instruction for both halves, each half rounded as the scalar
+// instruction rounds).  Multiply-adds are written out: nothing is contracted
+// across the packed instructions.
+struct F2 {
+    unsigned long long v;
 };
-
-__device__ __forceinline__ float dv_diff32(const MeanF &m, int model, int fld, float a, float b) {
-    const float pb = m.pb;
-    const float C = m.cb + b;
-    if (model == MODEL_QUADRATIC) {
-        // V' = phi + C1 chi^2 phi ; V'_chi = C1 phi^2 chi
-        if (fld == 0) return a + m.q0 * (pb * b * (m.cb2 + b) + a * C * C);
-        return m.q0 * (a * (m.pb2 + a) * C + m.pbsq * b);
-    }
-    // V' = lam phi^3 + g chi^2 phi ; V'_chi = g phi^2 chi
-    if (fld == 0) return m.q0 * a * (m.pb3sq + a * (3.f * pb + a)) + m.q1 * (pb * b * (m.cb2 + b) + a * C * C);
-    return m.q1 * (a * (m.pb2 + a) * C + m.pbsq * b);
+__device__ __forceinline__ F2 f2(float x, float y) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ F2 f2(float x) { return f2(x, x); }
+__device__ __forceinline__ float2 unpack(F2 a) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v));
+    return r;
+}
+__device__ __forceinline__ F2 operator+(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 operator*(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ F2 operator-(F2 a, F2 b) { return fma2(b, f2(-1.f), a); }
+__device__ __forceinline__ double sum2(F2 a) {
+    const float2 r = unpack(a);
+    return (double)r.x + (double)r.y;
 }
 
-__device__ __forceinline__ float v_diff32(const MeanF &m, int model, float a, float b) {
-    const float pb = m.pb, cb = m.cb;
-    const float P = pb + a, C = cb + b;
-    const float cross = (pb * b + cb * a + a * b) * (P * C + pb * cb);
-    if (model == MODEL_QUADRATIC) return a * (pb + 0.5f * a) + m.q1 * cross;
-    return m.q2 * a * (4.f * pb * pb * pb + a * (6.f * pb * pb + a * (4.f * pb + a))) + m.q3 * cross;
+// The homogeneous values and model constants as pairs, as the site functions
+// use them.
+struct alignas(16) MeanP {
+    F2 pb, cb, cb2, pb2, pbsq, pbcb;    // phi, chi, 2 chi, 2 phi, phi^2, phi chi
+    F2 pbt, pb3sq;                      // 3 phi, 3 phi^2
+    F2 pb4, pb6sq, pb4cu, pad;          // 4 phi, 6 phi^2, 4 phi^3
+};
+struct alignas(16) ModelP {
+    F2 n0, n1, q1, q2, q3, half;        // -mc[0], -mc[1], mc[1], mc[2], mc[3], 1/2
+};
+__device__ __forceinline__ MeanP mean_p(const double *fb) {
+    const double p = fb[0], c = fb[1];
+    auto k = [](double x) { return f2((float)x); };
+    return MeanP{k(p),      k(c),          k(2. * c),      k(2. * p),          k(p * p), k(p * c), k(3. * p),
+                 k(3. * p * p), k(4. * p), k(6. * p * p), k(4. * p * p * p), f2(0.f)};
+}
+__device__ __forceinline__ ModelP model_p(const LatticeConsts &c) {
+    auto k = [](double x) { return f2((float)x); };
+    return ModelP{k(-c.mc[0]), k(-c.mc[1]), k(c.mc[1]), k(c.mc[2]), k(c.mc[3]), f2(0.5f)};
+}
+
+// Takes V'(fbar+d) - V'(fbar) of both fields off t.
+__device__ __forceinline__ void sub_dv_diff32(const MeanP &m, const ModelP &q, int model, F2 a, F2 b, F2 (&t)[2]) {
+    const F2 C = m.cb + b;
+    const F2 u = fma2(a, C * C, (m.pb * b) * (m.cb2 + b));  // pb b (2 cb + b) + a C^2
+    const F2 w = fma2(a * (m.pb2 + a), C, m.pbsq * b);
+    if (model == MODEL_QUADRATIC) {
+        // V' = phi + C1 chi^2 phi ; V'_chi = C1 phi^2 chi
+        t[0] = fma2(q.n0, u, t[0] - a);
+        t[1] = fma2(q.n0, w, t[1]);
+    } else {
+        // V' = lam phi^3 + g chi^2 phi ; V'_chi = g phi^2 chi
+        t[0] = fma2(q.n0 * a, fma2(a, m.pbt + a, m.pb3sq), fma2(q.n1, u, t[0]));
+        t[1] = fma2(q.n1, w, t[1]);
+    }
+}
+
+// V(fbar+d) - V(fbar).
+__device__ __forceinline__ F2 v_diff32(const MeanP &m, const ModelP &q, int model, F2 a, F2 b) {
+    const F2 cross = fma2(a, b, fma2(m.cb, a, m.pb * b)) * fma2(m.pb + a, m.cb + b, m.pbcb);
+    if (model == MODEL_QUADRATIC) return fma2(q.q1, cross, a * fma2(q.half, a, m.pb));
+    const F2 quart = fma2(a, fma2(a, m.pb4 + a, m.pb6sq), m.pb4cu);
+    return fma2(q.q2 * a, quart, q.q3 * cross);
 }
 
 // Homogeneous potential and force in FP64 (for the FP32 path's mean).

@@ -78,7 +78,7 @@ __host__ __device__ constexpr int ens_tile_k(int shape) { return shape == 0 ? 64
 __host__ __device__ constexpr int ens_tile_j(int shape) { return shape == 0 ? 8 : 16; }
 template <int MODE>
 constexpr size_t ens_ring_bytes() {
-    constexpr int a = s32::Ring<32, 8, true>::SLOT, b = s32::Ring<16, 16, true>::SLOT, c = s32::Ring<8, 16, true>::SLOT;
+    constexpr int a = s32::Ring<32, 8>::SLOT, b = s32::Ring<16, 16>::SLOT, c = s32::Ring<8, 16>::SLOT;
     return sizeof(float) * ens_ring<MODE>() * (a > b ? (a > c ? a : c) : (b > c ? b : c));
 }
 
@@ -103,14 +103,16 @@ __global__ void __launch_bounds__(kEnsThreads, s32::sweep32_threads_per_sm<MODE>
     t.i0 = item.i0;
     t.i1 = item.i1;
     t.planes = 0;
-    const s32::Site32 s = s32::site32_consts<MODE>(c, L.sc);
+    __shared__ s32::Site32 s;
+    // by a warp that copies nothing; the march waits for the block before it reads them
+    if (tid == (int)blockDim.x - 1) s32::site32_consts<MODE>(c, L.sc, s);
     double acc[kNV];
 #pragma unroll
     for (int q = 0; q < kNV; q++) acc[q] = 0.;
     constexpr int S = ens_ring<MODE>();
-    if (item.shape == 0) s32::march32<32, 8, MODE, S, kEnsThreads, -1, true>(c, s, t, ring, acc);
-    else if (item.shape == 1) s32::march32<16, 16, MODE, S, kEnsThreads, -1, true>(c, s, t, ring, acc);
-    else s32::march32<8, 16, MODE, S, kEnsThreads, -1, true>(c, s, t, ring, acc);
+    if (item.shape == 0) s32::march32<32, 8, MODE, S, kEnsThreads>(c, s, t, ring, acc);
+    else if (item.shape == 1) s32::march32<16, 16, MODE, S, kEnsThreads>(c, s, t, ring, acc);
+    else s32::march32<8, 16, MODE, S, kEnsThreads>(c, s, t, ring, acc);
     if constexpr (MODE != MODE_B) {
         block_reduce<kNV>(acc, sred);
         if (tid == 0)

@@ -22,8 +22,8 @@ constexpr int ring_slots() {
 template <int TK2, int TJ, int MODE, int MODEL>
 static cudaError_t launch32m(const StencilArgs &a, dim3 grid, cudaStream_t s) {
     constexpr int S = ring_slots<MODE>();
-    auto k = s32::sweep32_kernel<TK2, TJ, MODE, S, MODEL, true>;
-    const size_t smem = (size_t)S * s32::Ring<TK2, TJ, true>::SLOT * sizeof(float);
+    auto k = s32::sweep32_kernel<TK2, TJ, MODE, S, MODEL>;
+    const size_t smem = (size_t)S * s32::Ring<TK2, TJ>::SLOT * sizeof(float);
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     k<<<grid, TK2 * TJ, smem, s>>>(a);

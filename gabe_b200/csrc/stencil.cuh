@@ -96,10 +96,6 @@ __device__ __forceinline__ double div_by(double x, const Divisor &v) {
 __device__ __forceinline__ double lap64(const Nb7<double> &f, const Divisor &dx2) {
     return div_by(f.v[1] + f.v[2] + f.v[3] + f.v[4] + f.v[5] + f.v[6] - 6. * f.v[0], dx2);
 }
-__device__ __forceinline__ float lap32(const Nb7<float> &f, float inv_dx2) {
-    return fmaf(-6.f, f.v[0], ((f.v[1] + f.v[2]) + (f.v[3] + f.v[4])) + (f.v[5] + f.v[6])) * inv_dx2;
-}
-
 // GW source components 11,12,13,22,23 of one field added into s
 // (jtg_stresstensor, g2evolutionpert.cpp:48-132, operation order kept).  The
 // source is traceless, so component 33 (= -11 - 22) is never stored: the
@@ -122,17 +118,16 @@ __device__ __forceinline__ void source_add64(const LatticeConsts &c, const Nb7<d
 // f(x + e_i) - f(x - e_i) are summed over both fields first (grad_prod_add),
 // then scaled once (source_from_prod): dn/4 (e_i e_j - delta_ij |e|^2 / 3),
 // the same tensor as source_add64 in fewer instructions.
-__device__ __forceinline__ void grad_prod_add(const Nb7<float> &f, float (&P)[6]) {
-    const float e1 = f.v[1] - f.v[2], e2 = f.v[3] - f.v[4], e3 = f.v[5] - f.v[6];
-    P[0] = fmaf(e1, e1, P[0]);
-    P[1] = fmaf(e2, e2, P[1]);
-    P[2] = fmaf(e3, e3, P[2]);
-    P[3] = fmaf(e1, e2, P[3]);
-    P[4] = fmaf(e1, e3, P[4]);
-    P[5] = fmaf(e2, e3, P[5]);
+__device__ __forceinline__ void grad_prod_add(F2 e1, F2 e2, F2 e3, F2 (&P)[6]) {
+    P[0] = fma2(e1, e1, P[0]);
+    P[1] = fma2(e2, e2, P[1]);
+    P[2] = fma2(e3, e3, P[2]);
+    P[3] = fma2(e1, e2, P[3]);
+    P[4] = fma2(e1, e3, P[4]);
+    P[5] = fma2(e2, e3, P[5]);
 }
-__device__ __forceinline__ void source_from_prod(float q /* dn / 4 */, const float (&P)[6], float *s) {
-    const float t = (1.f / 3.f) * ((P[0] + P[1]) + P[2]);
+__device__ __forceinline__ void source_from_prod(F2 q /* dn / 4 */, F2 third, const F2 (&P)[6], F2 (&s)[kSrc]) {
+    const F2 t = third * ((P[0] + P[1]) + P[2]);
     s[0] = q * (P[0] - t);
     s[1] = q * P[3];
     s[2] = q * P[4];
@@ -157,21 +152,6 @@ __device__ __forceinline__ MeanTraj mean_traj(const LatticeConsts &c, const DevS
     return m;
 }
 
-__device__ __forceinline__ MeanF mean_f(const LatticeConsts &c, const double *fb) {
-    MeanF m;
-    m.pb = (float)fb[0];
-    m.cb = (float)fb[1];
-    m.q0 = (float)c.mc[0];
-    m.q1 = (float)c.mc[1];
-    m.q2 = (float)c.mc[2];
-    m.q3 = (float)c.mc[3];
-    m.pb2 = (float)(2. * fb[0]);
-    m.cb2 = (float)(2. * fb[1]);
-    m.pbsq = (float)(fb[0] * fb[0]);
-    m.pb3sq = (float)(3. * fb[0] * fb[0]);
-    return m;
-}
-
 // FP32 energy sums (the FP32 sweeps here and in sweep32.cuh).
 // Reduced values of sweep A / E0 are sums over sites of expressions such as
 // (dfbar + d)^2 whose large homogeneous parts are known per launch.  Each
@@ -181,18 +161,18 @@ __device__ __forceinline__ MeanF mean_f(const LatticeConsts &c, const double *fb
 //   sum (dfbar + d)^2 = n dfbar^2 + 2 dfbar sum d + sum d^2,
 // so no site needs an FP32 -> FP64 conversion (that conversion pipe, not
 // HBM, bounded the per-site FP64 form).
-constexpr int kGroup = 8;
-struct Moments {
-    float a[2];  // sum d (momentum fluctuation) per field
-    float b;     // sum over fields of d^2
-    float c[2];  // sum Pd per field (stage-1 momentum before the adot0 term)
-    float e;     // sum over fields of Pd^2
-    float f;     // sum over fields of Pd d
-    float g0, g1;  // sum over fields of f lap f, stage 0 and stage 1
-    float v0, v1;  // potential differences, stage 0 and stage 1
+constexpr int kGroup = 16;
+struct Moments {     // each of the thread's even and odd sites apart
+    F2 a[2];         // sum d (momentum fluctuation) per field
+    F2 b;            // sum over fields of d^2
+    F2 c[2];         // sum Pd per field (stage-1 momentum before the adot0 term)
+    F2 e;            // sum over fields of Pd^2
+    F2 f;            // sum over fields of Pd d
+    F2 g0, g1;       // sum over fields of f dx^2 lap f, stage 0 and stage 1
+    F2 v0, v1;       // potential differences, stage 0 and stage 1
 };
 __device__ __forceinline__ void zero(Moments &m) {
-    m.a[0] = m.a[1] = m.b = m.c[0] = m.c[1] = m.e = m.f = m.g0 = m.g1 = m.v0 = m.v1 = 0.f;
+    m.a[0] = m.a[1] = m.b = m.c[0] = m.c[1] = m.e = m.f = m.g0 = m.g1 = m.v0 = m.v1 = f2(0.f);
 }
 
 // Folds the moments of n sites into the FP64 sums kin0 pot0 grad0 | pot1
@@ -201,20 +181,21 @@ __device__ __forceinline__ void zero(Moments &m) {
 // sum PQ = n pbar qbar + pbar q3 sum d + qbar sum Pd + q3 sum Pd d,
 // sum Q^2 = n qbar^2 + 2 qbar q3 sum d + q3^2 sum d^2.
 template <int MODE>
-__device__ __forceinline__ void fold(const MeanTraj &t, float q3f, int n, Moments &m, double (&acc)[kNV]) {
-    const double dn = (double)n, q3 = (double)q3f;
-    const double a0 = m.a[0], a1 = m.a[1], b = m.b;
+__device__ __forceinline__ void fold(const MeanTraj &t, double q3, double inv_dx2, int n, Moments &m,
+                                     double (&acc)[kNV]) {
+    const double dn = (double)n;
+    const double a0 = sum2(m.a[0]), a1 = sum2(m.a[1]), b = sum2(m.b);
     acc[0] += dn * (t.dfb0[0] * t.dfb0[0] + t.dfb0[1] * t.dfb0[1]) + 2. * (t.dfb0[0] * a0 + t.dfb0[1] * a1) + b;
-    acc[1] += (double)m.v0;
-    acc[2] -= (double)m.g0;
+    acc[1] += sum2(m.v0);
+    acc[2] -= inv_dx2 * sum2(m.g0);
     if constexpr (MODE != MODE_E0) {
-        const double c0 = m.c[0], c1 = m.c[1];
-        acc[3] += (double)m.v1;
-        acc[4] -= (double)m.g1;
+        const double c0 = sum2(m.c[0]), c1 = sum2(m.c[1]);
+        acc[3] += sum2(m.v1);
+        acc[4] -= inv_dx2 * sum2(m.g1);
         acc[5] += dn * (t.pbar[0] * t.pbar[0] + t.pbar[1] * t.pbar[1]) + 2. * (t.pbar[0] * c0 + t.pbar[1] * c1) +
-                  (double)m.e;
+                  sum2(m.e);
         acc[6] += dn * (t.pbar[0] * t.qbar[0] + t.pbar[1] * t.qbar[1]) + q3 * (t.pbar[0] * a0 + t.pbar[1] * a1) +
-                  (t.qbar[0] * c0 + t.qbar[1] * c1) + q3 * (double)m.f;
+                  (t.qbar[0] * c0 + t.qbar[1] * c1) + q3 * sum2(m.f);
         acc[7] += dn * (t.qbar[0] * t.qbar[0] + t.qbar[1] * t.qbar[1]) + 2. * q3 * (t.qbar[0] * a0 + t.qbar[1] * a1) +
                   q3 * q3 * b;
     }

@@ -7,12 +7,23 @@
 //   * a block owns a TK x TJ column tile (TK = 2 TK2 along k, two sites per
 //     thread, 8-byte accesses) and marches along i over `ci` planes;
 //   * every plane of the four input arrays (f phi, f chi, fdot phi, fdot chi)
-//     -- the thread's own pair of sites plus the one-point j/k halo -- is
-//     copied global -> shared with cp.async into a ring of S plane slots, S-3
-//     planes ahead of the plane being computed, so each thread keeps three
-//     planes of 8-byte loads in flight without holding them in registers;
+//     -- the tile plus the one-point j/k halo -- is copied global -> shared
+//     with cp.async, one 16-byte chunk per thread and array, into a ring of S
+//     plane slots, S-3 planes ahead of the plane being computed;
 //   * one barrier per plane: the slot of plane i-2 is refilled (plane i+S-2)
-//     only after every thread has left plane i-1.
+//     only after every thread has left plane i-1;
+//   * a thread's two sites are one packed value (F2): sm_100's packed FP32
+//     units take both with one instruction;
+//   * the planes are walked three at a turn, so that the own pairs of planes
+//     i-1, i, i+1 change roles instead of registers, and the constants lie in
+//     shared memory.
+// The sweeps were bound by instruction issue, not by HBM: with one site per
+// instruction, the neighbours' stage-1 values formed one by one, separate own
+// and halo copies and the constants in registers a warp took 424 instructions
+// per plane of sweep A (370 sweep B), now 210 (188).  At 256^3, fields only:
+// sweep A 118 against 152 us, B 111 against 119 (its 537 MB take 82 at the
+// measured copy rate), energies alone 107 against 118.  With GW sources the
+// stores bound sweep A.
 // Each input value crosses HBM once per sweep (halo points are re-read from
 // L2 by the neighbouring tiles).
 #pragma once
@@ -27,13 +38,8 @@ __device__ __forceinline__ void cp_async8(void *smem, const void *gmem) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
 }
 // 16 bytes, cached in L2 only.
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+__device__ __forceinline__ void cp_async16(unsigned s, const void *gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async4(void *smem, const void *gmem) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int NPEND>
@@ -43,46 +49,49 @@ __device__ __forceinline__ void cp_wait() {
 
 // Shared-memory plane slot: [4 arrays][TJ + 2 rows][PK columns]; column C0-1
 // is the k0-1 halo, columns C0 .. C0+TK-1 the tile, column C0+TK the k0+TK
-// halo.  Narrow (W16 false): C0 = 2, PK = TK + 4, every thread's pair on an
-// 8-byte boundary, one 8-byte copy per thread.  Wide (W16): C0 = 4,
-// PK = TK + 8, rows 16-byte multiples, so the pairs of threads 2m and 2m+1
-// land as one 16-byte copy (L2 only).  The single-lattice and ensemble
-// sweeps use the wide slots (at 512^3 sweep A 1.81 ms against 1.83 narrow,
-// sweep B 0.835 with five wide slots against 0.87 with six narrow ones).
-template <int TK2, int TJ, bool W16 = false>
+// halo.  C0 = 4, PK = TK + 8: rows are 16-byte multiples, so every copy is one
+// of 16 bytes (L2 only): the pairs of threads 2m and 2m+1, four points of a
+// halo row, and a halo column's point with the three beside it, which nothing
+// reads.
+template <int TK2, int TJ>
 struct Ring {
-    static constexpr int TK = 2 * TK2, PK = TK + (W16 ? 8 : 4), ROWS = TJ + 2, C0 = W16 ? 4 : 2;
+    static constexpr int TK = 2 * TK2, PK = TK + 8, ROWS = TJ + 2, C0 = 4;
     static constexpr int ARR = ROWS * PK, SLOT = 4 * ARR;
 };
 
-// Per-launch constants of the FP32 site update (stage scalars as floats,
-// homogeneous trajectory).
-struct Site32 {
+// Per-launch constants of the FP32 site update (stage scalars as pairs,
+// homogeneous trajectory).  They lie in shared memory: read again at each
+// plane by a few broadcast loads, they leave the registers to the march.
+struct alignas(16) Site32 {
+    MeanP m0, m1;
+    ModelP q;
+    F2 h, dt, k0, k1, n3H0, n3H1, qs, third, m6, pad;  // k = 1 / (a dx)^2, n3H = -3 H of the stages, qs = dn / 4
     MeanTraj mt;
-    MeanF m0, m1;
-    float ia02f, ia12f, c3H0f, c3H1f, hf, dtf, inv_dx2f, qsf, q3f;  // qsf = dn / 4
+    double inv_dx2, q3;
 };
 
 template <int MODE>
-__device__ __forceinline__ Site32 site32_consts(const LatticeConsts &c, const DevScalars *scp) {
-    Site32 s{};
+__device__ __forceinline__ void site32_consts(const LatticeConsts &c, const DevScalars *scp, Site32 &s) {
     const double h = c.half_dt, a0 = scp->a[0];
+    auto k = [](double x) { return f2((float)x); };
     s.mt = mean_traj(c, scp);
-    s.m0 = mean_f(c, s.mt.fb0);
-    s.m1 = mean_f(c, s.mt.fb1);
-    s.ia02f = (float)(1.0 / (a0 * a0));
-    s.hf = (float)h;
-    s.dtf = (float)c.dt;
-    s.inv_dx2f = (float)(1.0 / c.inv_dx2_div);
-    s.qsf = (float)(0.25 * c.dn);
-    s.q3f = (float)(-h * 3. / a0);
+    s.m0 = mean_p(s.mt.fb0);
+    s.m1 = mean_p(s.mt.fb1);
+    s.q = model_p(c);
+    s.inv_dx2 = 1.0 / c.inv_dx2_div;
+    s.q3 = (double)(float)(-h * 3. / a0);
+    s.h = k(h);
+    s.dt = k(c.dt);
+    s.k0 = k(s.inv_dx2 / (a0 * a0));
+    s.qs = k(0.25 * c.dn);
+    s.third = f2(1.f / 3.f);
+    s.m6 = f2(-6.f);
     if constexpr (MODE == MODE_B) {
         const double ad0 = scp->adot[0], a1 = scp->a[1], ad1 = scp->adot[1];
-        s.ia12f = (float)(1.0 / (a1 * a1));
-        s.c3H0f = (float)((3. * ad0) / a0);
-        s.c3H1f = (float)((3. * ad1) / a1);
+        s.k1 = k(s.inv_dx2 / (a1 * a1));
+        s.n3H0 = k(-(3. * ad0) / a0);
+        s.n3H1 = k(-(3. * ad1) / a1);
     }
-    return s;
 }
 
 // Potential of the site functions: MODEL >= 0 fixes it at compile time (the
@@ -93,64 +102,91 @@ __device__ __forceinline__ int site_model(const LatticeConsts &c) {
     return MODEL >= 0 ? MODEL : c.model;
 }
 
-// One site of sweep A / E0: adds to the moments, fills the sources.
+// What the site functions take of one array at the thread's pair of sites:
+// the values, dx^2 times the Laplacian and the undivided central differences.
+// The stage-1 fields are f + h fdot, so these of stage 1 follow from f's and
+// fdot's without forming the neighbours' stage-1 values.
+struct Pair {
+    F2 v, lap, e[3];
+};
+// own pairs of planes i, i+1, i-1 and rows j+1, j-1; the points left and right of the pair
+template <bool GRAD>
+__device__ __forceinline__ Pair pair_of(F2 m6, F2 cu, F2 nx, F2 pr, F2 up, F2 dn, float lm, float rp) {
+    Pair p;
+    p.v = cu;
+    const float2 c = unpack(cu);
+    p.lap = fma2(m6, cu, ((nx + pr) + (up + dn)) + f2(c.y + lm, rp + c.x));
+    if constexpr (GRAD) {
+        p.e[0] = nx - pr;
+        p.e[1] = up - dn;
+        p.e[2] = f2(c.y - lm, rp - c.x);
+    }
+    return p;
+}
+
+// The thread's pair of sites in sweep A / E0: adds to the moments, fills the sources.
 template <int MODE, int MODEL = -1>
-__device__ __forceinline__ void site_a32(const LatticeConsts &c, const Site32 &s, const Nb7<float> &fp,
-                                         const Nb7<float> &fc, const Nb7<float> &dp, const Nb7<float> &dc,
-                                         Moments &m, float (&s0)[kSrc], float (&s1)[kSrc]) {
+__device__ __forceinline__ void site_a32(const LatticeConsts &c, const Site32 &s, const Pair (&p)[4], Moments &m,
+                                         F2 (&s0)[kSrc], F2 (&s1)[kSrc]) {
     const int model = site_model<MODEL>(c);
-    const Nb7<float> *f0[2] = {&fp, &fc}, *d0[2] = {&dp, &dc};
-    float f1c[2];
-    float P0[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, P1[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    const F2 h = s.h;
+    F2 t0[2] = {s.k0 * p[0].lap, s.k0 * p[1].lap}, f1[2];  // stage-0 force without the drag
+    if constexpr (MODE != MODE_E0) sub_dv_diff32(s.m0, s.q, model, p[0].v, p[1].v, t0);
+    F2 P0[6], P1[6];
+    if constexpr (MODE == MODE_A_GW) {
+#pragma unroll
+        for (int q = 0; q < 6; q++) P0[q] = P1[q] = f2(0.f);
+    }
 #pragma unroll
     for (int f = 0; f < 2; f++) {
-        const Nb7<float> &ff = *f0[f], &dd = *d0[f];
-        const float lap0 = lap32(ff, s.inv_dx2f);
-        const float d = dd.v[0];
-        m.a[f] += d;
-        m.b = fmaf(d, d, m.b);
-        m.g0 = fmaf(ff.v[0], lap0, m.g0);
+        const Pair &ff = p[f], &dd = p[2 + f];
+        const F2 d = dd.v;
+        m.a[f] = m.a[f] + d;
+        m.b = fma2(d, d, m.b);
+        m.g0 = fma2(ff.v, ff.lap, m.g0);
         if constexpr (MODE != MODE_E0) {
-            const Nb7<float> f1 = axpy7(ff, s.hf, dd);
-            f1c[f] = f1.v[0];
-            const float Pd = d + s.hf * (lap0 * s.ia02f - dv_diff32(s.m0, model, f, fp.v[0], fc.v[0]));
-            m.c[f] += Pd;
-            m.e = fmaf(Pd, Pd, m.e);
-            m.f = fmaf(Pd, d, m.f);
-            m.g1 = fmaf(f1.v[0], lap32(f1, s.inv_dx2f), m.g1);
+            f1[f] = fma2(h, d, ff.v);
+            const F2 Pd = fma2(h, t0[f], d);
+            m.c[f] = m.c[f] + Pd;
+            m.e = fma2(Pd, Pd, m.e);
+            m.f = fma2(Pd, d, m.f);
+            m.g1 = fma2(f1[f], fma2(h, dd.lap, ff.lap), m.g1);
             if constexpr (MODE == MODE_A_GW) {
-                grad_prod_add(ff, P0);
-                grad_prod_add(f1, P1);
+                grad_prod_add(ff.e[0], ff.e[1], ff.e[2], P0);
+                grad_prod_add(fma2(h, dd.e[0], ff.e[0]), fma2(h, dd.e[1], ff.e[1]), fma2(h, dd.e[2], ff.e[2]), P1);
             }
         }
     }
     if constexpr (MODE == MODE_A_GW) {
-        source_from_prod(s.qsf, P0, s0);
-        source_from_prod(s.qsf, P1, s1);
+        source_from_prod(s.qs, s.third, P0, s0);
+        source_from_prod(s.qs, s.third, P1, s1);
     }
-    m.v0 += v_diff32(s.m0, model, fp.v[0], fc.v[0]);
-    if constexpr (MODE != MODE_E0) m.v1 += v_diff32(s.m1, model, f1c[0], f1c[1]);
+    m.v0 = m.v0 + v_diff32(s.m0, s.q, model, p[0].v, p[1].v);
+    if constexpr (MODE != MODE_E0) m.v1 = m.v1 + v_diff32(s.m1, s.q, model, f1[0], f1[1]);
 }
 
-// One site of sweep B: the new field and momentum of both fields.
+// The pair in sweep B: the new field and momentum of both fields.
 template <int MODEL = -1>
-__device__ __forceinline__ void site_b32(const LatticeConsts &c, const Site32 &s, const Nb7<float> &fp,
-                                         const Nb7<float> &fc, const Nb7<float> &dp, const Nb7<float> &dc,
-                                         float (&xo)[2], float (&dout)[2]) {
+__device__ __forceinline__ void site_b32(const LatticeConsts &c, const Site32 &s, const Pair (&p)[4], F2 (&xo)[2],
+                                         F2 (&dout)[2]) {
     const int model = site_model<MODEL>(c);
-    const Nb7<float> *f0[2] = {&fp, &fc}, *d0[2] = {&dp, &dc};
-    const Nb7<float> f1[2] = {axpy7(fp, s.hf, dp), axpy7(fc, s.hf, dc)};
+    const F2 h = s.h, dt = s.dt;
+    F2 t0[2], t1[2], f1[2], d1[2];
 #pragma unroll
     for (int f = 0; f < 2; f++) {
-        const Nb7<float> &ff = *f0[f], &dd = *d0[f];
-        const float lap0 = lap32(ff, s.inv_dx2f);
-        const float dd0 = lap0 * s.ia02f - dv_diff32(s.m0, model, f, fp.v[0], fc.v[0]) - s.c3H0f * dd.v[0];
-        const float d1c = dd.v[0] + s.hf * dd0;
-        const float lap1 = lap32(f1[f], s.inv_dx2f);
-        const float dd1 = lap1 * s.ia12f - dv_diff32(s.m1, model, f, f1[0].v[0], f1[1].v[0]) - s.c3H1f * d1c;
-        xo[f] = ff.v[0] + s.dtf * d1c;
-        dout[f] = dd.v[0] + s.dtf * dd1;
+        t0[f] = fma2(s.n3H0, p[2 + f].v, s.k0 * p[f].lap);
+        f1[f] = fma2(h, p[2 + f].v, p[f].v);
     }
+    sub_dv_diff32(s.m0, s.q, model, p[0].v, p[1].v, t0);
+#pragma unroll
+    for (int f = 0; f < 2; f++) {
+        d1[f] = fma2(h, t0[f], p[2 + f].v);
+        xo[f] = fma2(dt, d1[f], p[f].v);
+        t1[f] = fma2(s.n3H1, d1[f], s.k1 * fma2(h, p[2 + f].lap, p[f].lap));
+    }
+    sub_dv_diff32(s.m1, s.q, model, f1[0], f1[1], t1);
+#pragma unroll
+    for (int f = 0; f < 2; f++) dout[f] = fma2(dt, t1[f], p[2 + f].v);
 }
 
 // Threads per SM the register budget is sized for: sweep A with sources holds
@@ -174,14 +210,15 @@ struct Tile32 {
 // threads (NT >= TK2 TJ; threads beyond TK2 TJ only take part in the
 // barriers).  Sweep A / E0 add the tile's folded sums to acc (per-thread
 // partials, zero on idle threads); sweep B writes the new state.
-template <int TK2, int TJ, int MODE, int S, int NT, int MODEL = -1, bool W16 = false>
+template <int TK2, int TJ, int MODE, int S, int NT, int MODEL = -1>
 __device__ __forceinline__ void march32(const LatticeConsts &c, const Site32 &s, const Tile32 &t, float *ring,
                                         double (&acc)[kNV]) {
-    using Rg = Ring<TK2, TJ, W16>;
+    using Rg = Ring<TK2, TJ>;
     constexpr int TK = Rg::TK, PK = Rg::PK, C0 = Rg::C0;
     static_assert(S >= 4, "ring needs planes i-1, i, i+1 and one in flight");
-    static_assert(!W16 || TK2 % 2 == 0, "wide slots copy the pairs of threads 2m and 2m+1 of one row together");
-    static_assert(TK2 * TJ >= 2 * TK2 + 2 * TJ, "enough threads for the halo copies");
+    // chunks of 16 bytes of a plane's tile with its halo, one per thread and array
+    constexpr int CQ = TK / 4 + 2, CHUNKS = (TJ + 2) * CQ;
+    static_assert(TK % 4 == 0 && CHUNKS <= NT, "one chunk per thread");
     static_assert(NT >= TK2 * TJ, "block smaller than the tile");
     const int N = c.N;
     const int n3 = (t.planes ? t.planes : N) * N * N;  // < 2^31 for N <= 1024
@@ -190,48 +227,29 @@ __device__ __forceinline__ void march32(const LatticeConsts &c, const Site32 &s,
     const int tx = tid % TK2, ty = tid / TK2;
     const int k0 = t.k0, j0 = t.j0, i0 = t.i0, i1 = t.i1;
     const int j = j0 + ty, k = k0 + 2 * tx;
-    const float *src[4] = {t.X, t.X + n3, t.D, t.D + n3};
 
-    // element offsets of the own pair and the halo points within a plane;
-    // planes are p N^2
+    // the thread's own pair and the chunk that it copies (row cr, chunk cq; the
+    // corners are not read), as offsets within a plane; planes are p N^2
     const int NN = N * N;
-    const int jm = wrapi(j0 - 1, N), jp = wrapi(j0 + TJ, N), km = wrapi(k0 - 1, N), kp = wrapi(k0 + TK, N);
     const int o_own = j * N + k;
     const int so_own = (ty + 1) * PK + C0 + 2 * tx;  // shared offset of the own pair within an array
-    // halo duty, one copy per array: threads 0 .. 2 TK2 - 1 copy pairs of the
-    // j0-1 and j0+TJ rows, the next 2 TJ threads single points of the k0-1 and
-    // k0+TK columns
-    int h_kind = 0, h_so = 0, h_go = 0;  // 0 none, 8 pair, 4 point
-    if (tid < 2 * TK2) {
-        const int r = tid / TK2, q = tid % TK2;
-        h_kind = 8;
-        h_so = (r ? (TJ + 1) * PK : 0) + C0 + 2 * q;
-        h_go = (r ? jp : jm) * N + k0 + 2 * q;
-    } else if (tid < 2 * TK2 + 2 * TJ) {
-        const int r = (tid - 2 * TK2) / TJ, q = (tid - 2 * TK2) % TJ;
-        h_kind = 4;
-        h_so = (q + 1) * PK + (r ? TK + C0 : C0 - 1);
-        h_go = (j0 + q) * N + (r ? kp : km);
-    }
+    const int cr = tid / CQ, cq = tid % CQ;
+    const bool inner_r = cr > 0 && cr <= TJ, inner_q = cq > 0 && cq < CQ - 1;
+    const bool inner = tid < CHUNKS && inner_r && inner_q, copies = tid < CHUNKS && (inner_r || inner_q);
+    int ck = k0 - 4 + 4 * cq;
+    ck += ck < 0 ? N : (ck >= N ? -N : 0);
+    const int c_go = wrapi(j0 - 1 + cr, N) * N + ck;
+    const unsigned c_so = (unsigned)__cvta_generic_to_shared(ring + cr * PK + 4 * cq);
     auto issue = [&](int p, int sl) {  // plane p (wrapped) into slot sl
-        if (!act) return;
-        float *slot = ring + sl * Rg::SLOT;
-        const int pb = (t.planes ? p : wrapi(p, N)) * NN;
-#pragma unroll
-        for (int a = 0; a < 4; a++) {
-            float *sa = slot + a * Rg::ARR;
-            const float *g = src[a] + pb;
-            if constexpr (W16) {
-                // the pairs of threads 2m and 2m+1 as one 16-byte copy (k0 + 4m is 16-byte aligned)
-                if ((tx & 1) == 0) cp_async16(sa + so_own, g + o_own);
-            } else {
-                cp_async8(sa + so_own, g + o_own);
-            }
-            // the energies-only sweep reads the momenta at the own sites only
-            if (MODE == MODE_E0 && a >= 2) continue;
-            if (h_kind == 8) cp_async8(sa + h_so, g + h_go);
-            else if (h_kind == 4) cp_async4(sa + h_so, g + h_go);
-        }
+        if (!copies) return;
+        const unsigned d = c_so + sl * (unsigned)(Rg::SLOT * sizeof(float));
+        const int g = (t.planes ? p : wrapi(p, N)) * NN + c_go;
+        cp_async16(d, t.X + g);
+        cp_async16(d + Rg::ARR * 4, t.X + n3 + g);
+        // the energies-only sweep reads the momenta at the own sites only
+        if (MODE == MODE_E0 && !inner) return;
+        cp_async16(d + Rg::ARR * 8, t.D + g);
+        cp_async16(d + Rg::ARR * 12, t.D + n3 + g);
     };
     auto next_slot = [](int sl) { return sl + 1 == S ? 0 : sl + 1; };
 
@@ -246,90 +264,79 @@ __device__ __forceinline__ void march32(const LatticeConsts &c, const Site32 &s,
         if (p <= i1) issue(p, q);
         cp_commit();
     }
-    // slots of planes i-1, i, i+1 and of the plane issued next (i+S-2)
-    int s_pr = 0, s_cu = 1, s_nx = 2, s_is = S - 1;
-    float2 pr[4], cu[4];  // own pair of planes i-1 and i
     // sources [10][planes][N][N+2]: the whole lattice, or a slab's own planes (plane i at i - 1)
     const int splanes = t.planes ? t.planes - 2 : N, sfirst = t.planes ? 1 : 0;
     const int sstride = splanes * N * (N + 2);  // one source component
     const int so_row = j * (N + 2) + k;
-    for (int i = i0; i < i1; i++) {
+    using Own = F2[4];  // the own pair of the four arrays in one plane
+    auto own = [&](int sl, int a) {
+        return *reinterpret_cast<const F2 *>(ring + sl * Rg::SLOT + a * Rg::ARR + so_own);
+    };
+    int i = i0, s_cu = 1, s_nx = 2, s_is = S - 1;  // slots of planes i, i+1 and of the plane issued next (i+S-2)
+    // one plane: pr, cu are the own pairs of planes i-1 and i, nx becomes that of i+1
+    auto plane = [&](Own &pr, Own &cu, Own &nx) {
         cp_wait<S - 4>();  // planes up to i+1 have landed (this thread's copies)
         __syncthreads();   // ... and everybody's; every thread has left plane i-1
         if (i + S - 2 <= i1) issue(i + S - 2, s_is);  // into the slot of plane i-2
         cp_commit();
-
         if (act) {
-            const float *sc = ring + s_cu * Rg::SLOT;
-            const float *sn = ring + s_nx * Rg::SLOT;
-            if (i == i0) {
-                const float *sp = ring + s_pr * Rg::SLOT;
-#pragma unroll
-                for (int a = 0; a < 4; a++) {
-                    pr[a] = *reinterpret_cast<const float2 *>(sp + a * Rg::ARR + so_own);
-                    cu[a] = *reinterpret_cast<const float2 *>(sc + a * Rg::ARR + so_own);
-                }
-            }
-            Nb7<float> nb[4][2];  // [array][site]
-            float2 nx[4];
+            const float *sc = ring + s_cu * Rg::SLOT + so_own;
+            Pair p[4];
 #pragma unroll
             for (int a = 0; a < 4; a++) {
-                const int ao = a * Rg::ARR + so_own;
-                nx[a] = *reinterpret_cast<const float2 *>(sn + ao);
-                const float2 up = *reinterpret_cast<const float2 *>(sc + ao + PK);
-                const float2 dn = *reinterpret_cast<const float2 *>(sc + ao - PK);
-                const float lm = sc[ao - 1], rp = sc[ao + 2];
-                // reference neighbour order: centre, i+1, i-1, j+1, j-1, k+1, k-1
-                nb[a][0] = Nb7<float>{{cu[a].x, nx[a].x, pr[a].x, up.x, dn.x, cu[a].y, lm}};
-                nb[a][1] = Nb7<float>{{cu[a].y, nx[a].y, pr[a].y, up.y, dn.y, rp, cu[a].x}};
+                nx[a] = own(s_nx, a);
+                if (MODE == MODE_E0 && a >= 2) {  // own momenta only
+                    p[a].v = cu[a];
+                    continue;
+                }
+                const float *q = sc + a * Rg::ARR;
+                p[a] = pair_of<MODE == MODE_A_GW>(s.m6, cu[a], nx[a], pr[a], *reinterpret_cast<const F2 *>(q + PK),
+                                                  *reinterpret_cast<const F2 *>(q - PK), q[-1], q[2]);
             }
             if constexpr (MODE == MODE_B) {
-                float xo[2][2], dout[2][2];  // [site][field]
-#pragma unroll
-                for (int v = 0; v < 2; v++) {
-                    site_b32<MODEL>(c, s, nb[0][v], nb[1][v], nb[2][v], nb[3][v], xo[v], dout[v]);
-                }
+                F2 xo[2], dout[2];
+                site_b32<MODEL>(c, s, p, xo, dout);
                 const int gx = i * NN + o_own;
-                __stcs(reinterpret_cast<float2 *>(t.Xo + gx), make_float2(xo[0][0], xo[1][0]));
-                __stcs(reinterpret_cast<float2 *>(t.Xo + n3 + gx), make_float2(xo[0][1], xo[1][1]));
-                __stcs(reinterpret_cast<float2 *>(t.Do + gx), make_float2(dout[0][0], dout[1][0]));
-                __stcs(reinterpret_cast<float2 *>(t.Do + n3 + gx), make_float2(dout[0][1], dout[1][1]));
+                __stcs(reinterpret_cast<float2 *>(t.Xo + gx), unpack(xo[0]));
+                __stcs(reinterpret_cast<float2 *>(t.Xo + n3 + gx), unpack(xo[1]));
+                __stcs(reinterpret_cast<float2 *>(t.Do + gx), unpack(dout[0]));
+                __stcs(reinterpret_cast<float2 *>(t.Do + n3 + gx), unpack(dout[1]));
             } else {
-                float s0[2][kSrc] = {}, s1[2][kSrc] = {};
-#pragma unroll
-                for (int v = 0; v < 2; v++) {
-                    site_a32<MODE, MODEL>(c, s, nb[0][v], nb[1][v], nb[2][v], nb[3][v], mom, s0[v], s1[v]);
-                }
+                F2 s0[kSrc], s1[kSrc];
+                site_a32<MODE, MODEL>(c, s, p, mom, s0, s1);
                 if (++ngroup == kGroup || i == i1 - 1) {
-                    fold<MODE>(s.mt, s.q3f, 2 * ngroup, mom, acc);
+                    fold<MODE>(s.mt, s.q3, s.inv_dx2, 2 * ngroup, mom, acc);
                     ngroup = 0;
                 }
                 if constexpr (MODE == MODE_A_GW) {
                     float *g = t.S + ((i - sfirst) * (N * (N + 2)) + so_row);
 #pragma unroll
-                    for (int q = 0; q < kSrc; q++, g += sstride)
-                        __stcs(reinterpret_cast<float2 *>(g), make_float2(s0[0][q], s0[1][q]));
+                    for (int q = 0; q < kSrc; q++, g += sstride) __stcs(reinterpret_cast<float2 *>(g), unpack(s0[q]));
 #pragma unroll
-                    for (int q = 0; q < kSrc; q++, g += sstride)
-                        __stcs(reinterpret_cast<float2 *>(g), make_float2(s1[0][q], s1[1][q]));
+                    for (int q = 0; q < kSrc; q++, g += sstride) __stcs(reinterpret_cast<float2 *>(g), unpack(s1[q]));
                 }
             }
-#pragma unroll
-            for (int a = 0; a < 4; a++) {
-                pr[a] = cu[a];
-                cu[a] = nx[a];
-            }
         }
-        s_pr = s_cu;
         s_cu = s_nx;
         s_nx = next_slot(s_nx);
         s_is = next_slot(s_is);
+        return ++i < i1;
+    };
+    cp_wait<S - 3>();  // planes i0-1 and i0
+    __syncthreads();
+    Own x[3];
+    if (act) {
+#pragma unroll
+        for (int a = 0; a < 4; a++) x[0][a] = own(0, a), x[1][a] = own(1, a);
+    }
+    // three planes a turn, so that no pair moves from register to register
+    while (plane(x[0], x[1], x[2]) && plane(x[1], x[2], x[0]) && plane(x[2], x[0], x[1])) {
     }
     cp_wait<0>();
     __syncthreads();  // the ring may be refilled by the block's next tile
 }
 
-template <int TK2, int TJ, int MODE, int S, int MODEL = -1, bool W16 = false>
+template <int TK2, int TJ, int MODE, int S, int MODEL = -1>
 __global__ void __launch_bounds__(TK2 *TJ, (sweep32_threads_per_sm<MODE>() + TK2 * TJ - 1) / (TK2 * TJ))
     sweep32_kernel(StencilArgs args) {
     extern __shared__ __align__(16) float ring[];  // S slots
@@ -352,11 +359,13 @@ __global__ void __launch_bounds__(TK2 *TJ, (sweep32_threads_per_sm<MODE>() + TK2
     t.i0 = first + blockIdx.z * args.ci;
     t.i1 = min(t.i0 + args.ci, end);
 
-    const Site32 s = site32_consts<MODE>(c, args.sc);
+    __shared__ Site32 s;
+    // by a warp that copies nothing; the march waits for the block before it reads them
+    if (tid == (int)blockDim.x - 1) site32_consts<MODE>(c, args.sc, s);
     double acc[kNV];
 #pragma unroll
     for (int q = 0; q < kNV; q++) acc[q] = 0.;
-    march32<TK2, TJ, MODE, S, TK2 * TJ, MODEL, W16>(c, s, t, ring, acc);
+    march32<TK2, TJ, MODE, S, TK2 * TJ, MODEL>(c, s, t, ring, acc);
 
     const int bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
     if constexpr (MODE != MODE_B) {

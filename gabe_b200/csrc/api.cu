@@ -185,9 +185,9 @@ int source_fft(gabe_handle *h, int slot, cudaStream_t s) {
     }
     if (h->fftp) {  // the planes of the stage-0 and of the stage-1 sources, S -> S2; the lines run in the k-space update
         const int n = kSrc * h->N;
-        const size_t half = (size_t)kSrc * h->N * h->N * (h->N + 2);  // floats of one stage
+        const size_t in = (size_t)n * h->N * h->N, out = (size_t)n * h->N * (h->N + 2);  // floats of one stage
         for (int st = 0; st < 2; st++)
-            CK(h, fftp_planes_f32(h->N, static_cast<const float *>(S) + st * half, static_cast<float *>(h->S2) + st * half,
+            CK(h, fftp_planes_f32(h->N, static_cast<const float *>(S) + st * in, static_cast<float *>(h->S2) + st * out,
                                   n, s));
         return GABE_OK;
     }
@@ -228,6 +228,7 @@ StencilArgs stencil_args(gabe_handle *h, int cur, int slot = 0) {
     a.Do = h->D[1 - cur];
     a.S = source_buffer(h, slot);
     a.slot = slot;
+    a.tight = h->fftt || h->fftp;
     a.partials = h->partials;
     a.sc = h->sc;
     a.c = h->lc;
@@ -724,14 +725,14 @@ static int profile_fftt_passes(gabe_handle *h, int nreps, double ms_out[3]) {
         cudaError_t ce = cudaEventRecord(e[0], h->stream);
         const float *S = static_cast<const float *>(h->S);
         float *S2 = static_cast<float *>(h->S2);
-        const size_t half = (size_t)kSrc * h->N * h->N * (h->N + 2);
+        const size_t in = (size_t)kSrc * h->N * h->N * h->N, out = in + (size_t)kSrc * h->N * h->N * 2;
         unsigned int *st = &h->sc->status;
         if (ce == cudaSuccess)
             ce = h->fftp ? fftp_planes_f32(h->N, S, S2, kSrc * h->N, h->stream)
                          : fftt_rows_f32(h->N, S, S2, 2 * kSrc, st, h->stream);
         if (ce == cudaSuccess) ce = cudaEventRecord(e[1], h->stream);
         if (ce == cudaSuccess)
-            ce = h->fftp ? fftp_planes_f32(h->N, S + half, S2 + half, kSrc * h->N, h->stream)
+            ce = h->fftp ? fftp_planes_f32(h->N, S + in, S2 + out, kSrc * h->N, h->stream)
                          : fftt_cols_f32(h->N, h->S2, h->S, 2 * kSrc, st, h->stream);
         if (ce == cudaSuccess) ce = cudaEventRecord(e[2], h->stream);
         if (ce == cudaSuccess)

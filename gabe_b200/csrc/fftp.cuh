@@ -96,7 +96,7 @@ __device__ __forceinline__ void twiddles(float2 *tw) {
 template <int N>
 struct PlaneGeom {
     using C = Cfg<N>;
-    static constexpr int NH = N / 2 + 1, RP = N + 2, PR = N + 4;  // row pitch as stored, and in the work layout
+    static constexpr int NH = N / 2 + 1, RP = N, PR = N + 4;  // row pitch as stored, and in the work layout
     static constexpr int ROWS = C::PB * N, PAIRS = ROWS / 2;
     static constexpr size_t SMEM_BYTES = N * sizeof(float2) + (size_t)ROWS * PR * sizeof(float);
     static_assert(N % 16 == 0 && C::L1 * C::L2 == N && C::L1 % 2 == 0 && C::L2 % 2 == 0, "four-step split");
@@ -140,7 +140,8 @@ __global__ void __launch_bounds__(Cfg<N>::TP, Cfg<N>::MBP)
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         // rows, first step: L2-point DFTs over n2 (stride L1) of two neighbouring n1, twiddled,
         // from global memory to element k2 + L2 n1 of the work layout
-        const float *src = S + (size_t)tile * G::ROWS * RP;
+        // (the sources of one lattice after another stand 2 kSrc N^2 (N + 2) floats apart)
+        const float *src = S + (size_t)tile * G::ROWS * RP + (size_t)(tile / (2 * kSrc * N / PB)) * (2 * kSrc * N * N * 2);
         for (int t = tid; t < G::PAIRS * (L1 / 2); t += TP) {
             const int p = t / (L1 / 2), n1 = 2 * (t % (L1 / 2));
             const float *re = src + 2 * p * RP + n1, *im = re + RP;

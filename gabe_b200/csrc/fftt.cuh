@@ -43,9 +43,10 @@ using pfft::FourStep;
 // pass 1: rows along k -> T1[q][i][kz][j]
 // ---------------------------------------------------------------------------
 // A tile of 16 rows (8 pairs, each two real rows taken as one complex
-// sequence) is one contiguous run of 16 (N + 2) floats in S and lands in
-// shared memory by one bulk copy (cp.async.bulk + mbarrier) into a linear
-// buffer.  The four-step FFT's first pass reads the pairs from
+// sequence) is one contiguous run of S and lands in shared memory by one bulk
+// copy (cp.async.bulk + mbarrier); for N < 512 by one per row, N + L1 / 2
+// floats apart, so that the pairs that half a warp reads together start on
+// different banks (at 512 it reads of one pair).  The four-step FFT's first pass reads the pairs from
 // the linear buffer (lanes over consecutive elements: conflict-free) and
 // writes its output into a work buffer in the pair-preserving XOR swizzle of
 // fft3d.cuh, so that the second pass's stride-L1 reads fall on distinct
@@ -69,12 +70,13 @@ using pfft::FourStep;
 template <int N, int T_ = 128, int NB_ = 1>
 struct RowTGeom {
     using RG = f3d::RowGeom<N, 16, 1, T_, 2>;  // the work buffer (swizzled, pitch N + 2)
-    static constexpr int R = 16, RP = N + 2, NB = NB_;
+    static constexpr int R = 16, RP = RG::L1 == 32 ? N : N + RG::L1 / 2, NB = NB_;
     static constexpr size_t HEAD = 128;                          // NB mbarriers
     static constexpr size_t TW_BYTES = (size_t)N * sizeof(float2);  // twiddles of the four-step
     static constexpr size_t LIN_BYTES = (size_t)R * RP * sizeof(float);
     static constexpr size_t SMEM_BYTES = HEAD + TW_BYTES + NB * LIN_BYTES + (size_t)RG::BUF * sizeof(float);
     static_assert(LIN_BYTES % 16 == 0 && (HEAD + TW_BYTES) % 16 == 0, "bulk copies of 16-byte multiples");
+    static_assert(RP % 4 == 0, "every row lands on a 16-byte boundary");
 };
 
 template <int N, int T_ = 128, int MINB = 2, int NB_ = 1>
@@ -101,8 +103,11 @@ __global__ void __launch_bounds__(T_, MINB)
     int fills[NB] = {};  // thread 0: fills issued per buffer
     auto issue = [&](long long tile, int b) {
         fills[b]++;
-        tma::mbar_arrive_expect(&bar[b], (uint32_t)G::LIN_BYTES);
-        tma::load(lin0 + b * R * RP, S + tile * R * RP, (uint32_t)G::LIN_BYTES, &bar[b]);
+        tma::mbar_arrive_expect(&bar[b], (uint32_t)(R * N * sizeof(float)));
+        const float *src = S + tile * R * N;
+        if constexpr (RP == N) tma::load(lin0 + b * R * RP, src, (uint32_t)G::LIN_BYTES, &bar[b]);
+        else for (int r = 0; r < R; r++)
+            tma::load(lin0 + (b * R + r) * RP, src + r * N, (uint32_t)(N * sizeof(float)), &bar[b]);
     };
     if (tid == 0)
         for (int q = 0; q < NB; q++) {

@@ -9,11 +9,10 @@
 namespace gabe {
 
 // Plane slots of a sweep's ring (three planes being read, the rest in
-// flight), all in the wide layout (sweep32.cuh, Ring).  Measured at 512^3:
-// sweep A 1.81 ms with six slots (2.10 with four, 2.18 with ten); sweep B
-// 0.835 with five (0.87 with six narrow ones, 1.02 with four); the
-// energies-only sweep 0.2-0.4 with four against ~0.75 with six narrow ones.
-// Fewer slots leave more of the SM's shared memory to L1.
+// flight).  Measured at 512^3 with one site per instruction: sweep A 1.81 ms
+// with six slots (2.10 with four, 2.18 with ten); sweep B 0.835 with five
+// (1.02 with four); the energies-only sweep 0.2-0.4 with four against ~0.75
+// with six.  Fewer slots leave more of the SM's shared memory to L1.
 template <int MODE>
 constexpr int ring_slots() {
     return MODE == MODE_E0 ? 4 : (MODE == MODE_B ? 5 : 6);

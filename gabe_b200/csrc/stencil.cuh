@@ -63,6 +63,11 @@ struct StencilArgs {
     // Host memory (mapped) that receives the scalars after the last block has
     // finished the stage, or null: a caller that waits for them saves the copy.
     DevScalars *mirror;
+    // FP32 sources in rows of N reals instead of N + 2, for the transforms that work out of place (the plane and
+    // the transposed one; an in-place r2c needs the padding): each warp store is then two whole 128-byte lines
+    // instead of parts of three.  Sweep A at 512^3 1.39 ms against 1.70, at 128^3 37.4 us against 40.6; the plane
+    // pass at 128^3 64.7 us against 69.4, the transposed rows unchanged.
+    bool tight;
 };
 
 constexpr int kNV = 8;  // reduced values: kin0 pot0 grad0 | pot1 grad1 PP PQ QQ

@@ -4,10 +4,10 @@
 //   fields   X[buf][fld][i][j][k]     (k fastest; two ping-pong buffers)
 //   momenta  D[buf][fld][i][j][k]
 //   GW       h[12][i][j][kz], l[12][i][j][kz]   planar, kz < N/2+1
-//   sources  S[12][i][j][N+2]  real, padded rows so cuFFT can run R2C in
-//            place; afterwards the same bytes hold the 12 half-spectra
-//            S^[12][i][j][kz] (complex).  Slots 0..5 carry the stage-0
-//            source 11,12,13,22,23,33, slots 6..11 the stage-1 source.
+//   sources  S[10][i][j][row]  real: 11,12,13,22,23 of stage 0, then of
+//            stage 1; rows of N + 2 where the transform runs in place (the
+//            same bytes then hold the half spectra S^[10][i][j][kz]), of N
+//            where it writes a second array (FP32)
 //   scalars  DevScalars (a, adot, energies per stage, homogeneous
 //            trajectory of the FP32 path, status word)
 //   partials per-block FP64 sums of the energy reductions

@@ -102,15 +102,14 @@ inline GridPlan plan_grid32(int N, int want_shape, int want_ci) {
         return tk <= N && tj <= N && N % tk == 0 && N % tj == 0;
     };
     int shape = (want_shape >= 0 && want_shape < kNumShapes32 && fits(want_shape)) ? want_shape : -1;
-    // 128 x 4 columns at 512^3: sweep A 1.69 ms against 1.81 for 64 x 8 (sweep B 0.84 against 0.83)
-    if (shape < 0 && N == 512 && fits(2)) shape = 2;
     for (int q = 0; shape < 0 && q < kNumShapes32; q++)
         if (fits(q)) shape = q;
     if (shape < 0) return GridPlan{-1, 0, dim3(0, 0, 0)};  // no tile divides N (N % 16 != 0)
     const int TK = kShapes32[shape][0], TJ = kShapes32[shape][1];
     const int bxy = (N / TK) * (N / TJ);
-    // planes per block: N / 8 from N = 128 on (the fastest measured at 128^3, 256^3 and 512^3: 64 planes at
-    // 512^3 ran sweep A 1.69-1.81 ms against 1.97 with 128); below, enough blocks for four per SM
+    // planes per block: N / 8 from N = 128 on (the fastest measured at 128^3, 256^3 and 512^3, where 64 x 8
+    // columns of 64 planes take 2.23 ms for both sweeps, 128 x 4 2.30, 32 planes 2.32); below, enough blocks for four
+    // per SM
     int ci = want_ci > 0 ? want_ci : (N >= 128 ? N / 8 : N);
     if (want_ci <= 0 && N < 128)
         while (ci > 4 && (long long)bxy * ((N + ci - 1) / ci) < 4 * 148) ci /= 2;

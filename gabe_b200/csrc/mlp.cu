@@ -52,20 +52,17 @@ __device__ __forceinline__ bf16 cvt<bf16>(float v) { return __float2bfloat16_rn(
 
 __device__ __forceinline__ float sigmoid(float z) { return 1.f / (1.f + expf(-z)); }
 __device__ __forceinline__ float silu(float z) { return z * sigmoid(z); }
-// SiLU of the forward epilogues of the first-layer and tcgen05 kernels:
-// the fast exponential and division intrinsics (two special-function
-// operations per value, a few ulp of FP32, far below the BF16 rounding of
-// the stored activations), since the accurate expf and IEEE division
-// bounded those epilogues (608 against 185 us per 1M-row hidden layer).
-// A reciprocal by Newton-Raphson steps on the FMA pipe instead of the
-// second special-function operation measured slower (225 us): the
-// epilogue is bound by issue as much as by that pipe.  z -> -inf gives 0,
-// z -> +inf gives z.
-// Written with the flush-to-zero forms of the two operations: the plain
-// intrinsics guard against subnormal operands and results with three more
-// instructions each, which cannot matter here (1 + exp(-z) >= 1, and a
-// flushed exponential adds nothing to 1; a flushed reciprocal is the 0 that
-// the division intrinsic gives for such divisors).
+// SiLU of the forward epilogues of the first-layer and tcgen05 kernels, from
+// the identity exp(-z) = 2^(-z log2 e): z / (1 + 2^(-z log2 e)) on the
+// special-function unit's base-2 exponential and reciprocal (PTX ex2.approx
+// and rcp.approx, relative errors of at most 2^-22 and 2^-23), since expf and
+// an IEEE division bounded those epilogues (608 against 185 us per 1M-row
+// hidden layer).  Relative error at most 1.5 |z| 2^-24 (the rounded exponent)
+// + 2^-21, far below the BF16 rounding of the stored activations; a value
+// below |z| 2^-126 (z < -87) may be flushed to zero.  A reciprocal by
+// Newton-Raphson steps on the FMA pipe instead of the second special-function
+// operation measured slower (225 us): the epilogue is bound by issue as much
+// as by that pipe.
 __device__ __forceinline__ float silu_fast(float z) {
     float e, r;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(z * -1.4426950408889634f));

@@ -83,24 +83,28 @@ struct Nb7 {
 // correctly rounded quotient (Markstein's theorem; N. Brisebarre, J.-M.
 // Muller and S. K. Raina, "Accelerating correctly rounded floating-point
 // division when the divisor is known in advance", IEEE Trans. Computers 53
-// (2004)), so the reference's divisions keep their bits (finite quotients in
-// the normal range; an infinite numerator gives NaN instead of infinity).
-// The compiler's division, about four times the instructions, bounded the
-// FP64 sweeps: at 256^3 with GW sources sweep B takes 0.253 ms against 0.398
-// with it, sweep A 0.475 against 0.561 (32 x 4 columns, 32 planes per block).
+// (2004)), so the reference's divisions keep their bits where divisor,
+// quotient and residual are normal numbers (numerators below 2^-900, whose
+// residual underflows, are within an ulp).  The residual is taken with its
+// sign reversed, so that a zero numerator keeps its sign.  The residual of an
+// infinite quotient is NaN: sweep_kernel takes the states that have them
+// through sites_inf.  An ordinary division bounded the FP64 sweeps: at 256^3
+// with GW sources sweep B takes 0.253 ms against 0.398 with it, sweep A 0.475
+// against 0.561 (32 x 4 columns, 32 planes per block).
 struct Divisor {
     double d, r;
 };
 __device__ __forceinline__ Divisor divisor(double d) { return Divisor{d, 1.0 / d}; }
 __device__ __forceinline__ double div_by(double x, const Divisor &v) {
     const double q = x * v.r;
-    return fma(fma(-q, v.d, x), v.r, q);
+    return fma(-fma(q, v.d, -x), v.r, q);
 }
 
-// laplacian() of g2functions.cpp:35-43 in its operation order.
-__device__ __forceinline__ double lap64(const Nb7<double> &f, const Divisor &dx2) {
-    return div_by(f.v[1] + f.v[2] + f.v[3] + f.v[4] + f.v[5] + f.v[6] - 6. * f.v[0], dx2);
+// laplacian() of g2functions.cpp:35-43 in its operation order, times dx^2
+__device__ __forceinline__ double lap64(const Nb7<double> &f) {
+    return f.v[1] + f.v[2] + f.v[3] + f.v[4] + f.v[5] + f.v[6] - 6. * f.v[0];
 }
+__device__ __forceinline__ double lap64(const Nb7<double> &f, const Divisor &dx2) { return div_by(lap64(f), dx2); }
 // GW source components 11,12,13,22,23 of one field added into s
 // (jtg_stresstensor, g2evolutionpert.cpp:48-132, operation order kept).  The
 // source is traceless, so component 33 (= -11 - 22) is never stored: the
@@ -479,9 +483,73 @@ __device__ __forceinline__ void finish_b(const LatticeConsts &c, DevScalars *s) 
     s->step += 1;
 }
 
+// The sites (i0 .. i1-1, j, k) of a state that has blown up, divided by the operator and read from global memory:
+// what the march does for the other states, without its speed (sweep A's sources, which hold no quotient, are not
+// written again).  Out of line, on no local of the march and with little in registers, so that the march keeps its
+// own: a second march inlined beside the first cost sweep A at 256^3 without GW sources 276 us against 252, this
+// nothing (with sources 487 us against 512: 128 registers instead of 154).
+template <int MODE>
+__device__ __noinline__ void sites_inf(const StencilArgs &args, int i0, int i1, int j, int k, double *sums) {
+    const LatticeConsts &c = args.c;
+    const int N = c.N;
+    const size_t n3 = (size_t)(args.planes ? args.planes : N) * N * N;
+    const double *X = static_cast<const double *>(args.X), *D = static_cast<const double *>(args.D);
+    const double h = c.half_dt, dt = c.dt;
+    if constexpr (MODE != MODE_B)
+        for (int q = 0; q < kNV; q++) sums[q] = 0.;
+#pragma unroll 1
+    for (int i = i0; i < i1; i++) {
+        const size_t o = ((size_t)i * N + j) * N + k;
+        const double f00 = X[o], f01 = X[n3 + o], f10 = f00 + h * D[o], f11 = f01 + h * D[n3 + o];
+#pragma unroll 1
+        for (int f = 0; f < 2; f++) {
+            const double *x = X + f * n3, *d = D + f * n3;
+            double lap0 = 0., lap1 = 0.;
+#pragma unroll 1
+            for (int q = 1; q < 7; q++) {  // i+1, i-1, j+1, j-1, k+1, k-1
+                const int s = q & 1 ? 1 : -1;
+                const int ii = q > 2 ? i : (args.planes ? i + s : wrapi(i + s, N));
+                const int jj = (q + 1) / 2 == 2 ? wrapi(j + s, N) : j, kk = q > 4 ? wrapi(k + s, N) : k;
+                const size_t at = ((size_t)ii * N + jj) * N + kk;
+                const double v0 = x[at];
+                lap0 = q == 1 ? v0 : lap0 + v0;
+                if constexpr (MODE != MODE_E0) {
+                    const double v1 = v0 + h * d[at];
+                    lap1 = q == 1 ? v1 : lap1 + v1;
+                }
+            }
+            const double x0 = x[o], dx = d[o], x1 = x0 + h * dx, a0 = args.sc->a[0];
+            lap0 = (lap0 - 6. * x0) / c.inv_dx2_div;
+            lap1 = (lap1 - 6. * x1) / c.inv_dx2_div;
+            const double g = lap0 / a0 / a0 - dv64(c, f, f00, f01);
+            if constexpr (MODE == MODE_B) {
+                const double a1 = args.sc->a[1];
+                const double d1 = dx + h * (g - (3. * args.sc->adot[0]) / a0 * dx);
+                const double dd1 = lap1 / a1 / a1 - dv64(c, f, f10, f11) - (3. * args.sc->adot[1]) / a1 * d1;
+                static_cast<double *>(args.Xo)[f * n3 + o] = x0 + dt * d1;
+                static_cast<double *>(args.Do)[f * n3 + o] = dx + dt * dd1;
+            } else {
+                sums[0] += dx * dx;
+                sums[2] -= x0 * lap0;
+                if constexpr (MODE != MODE_E0) {
+                    const double P = dx + h * g, Q = -h * 3. * dx / a0;
+                    sums[4] -= x1 * lap1;
+                    sums[5] += P * P;
+                    sums[6] += P * Q;
+                    sums[7] += Q * Q;
+                }
+            }
+        }
+        if constexpr (MODE != MODE_B) {
+            sums[1] += pot64(c, f00, f01);
+            if constexpr (MODE != MODE_E0) sums[3] += pot64(c, f10, f11);
+        }
+    }
+}
+
 // Single lattice, FP64: block (x, y, z) = column tile (k, j) and plane chunk.
 template <typename T, int TK, int TJ, int MODE>
-__global__ void __launch_bounds__(TK *TJ) sweep_kernel(StencilArgs args) {
+__global__ void __launch_bounds__(TK *TJ) sweep_kernel(const __grid_constant__ StencilArgs args) {
     __shared__ __align__(16) T smem[2][4 * SweepSmem<TK, TJ>::P];
     __shared__ double sred[((TK * TJ + 31) / 32) * kNV];
     __shared__ int sflag;
@@ -502,9 +570,21 @@ __global__ void __launch_bounds__(TK *TJ) sweep_kernel(StencilArgs args) {
     double acc[kNV];
 #pragma unroll
     for (int q = 0; q < kNV; q++) acc[q] = 0.;
-    sweep_tile<T, TK, TJ, MODE>(c, job, smem[0], smem[1], acc);
-
     const int tid = threadIdx.x;
+    static_assert(sizeof(smem) >= TK * TJ * kNV * sizeof(double), "the tile buffers hold the sums of sites_inf");
+    double *sums = &smem[0][0] + tid * kNV;
+    // Infinite quotients make the state's energies infinite or NaN.  Sweep B knows that from sweep A; sweep A and the
+    // energies see it in their own sums.
+    if (MODE == MODE_B && (args.sc->status & ST_NONFINITE)) {
+        sites_inf<MODE>(args, job.i0, job.i1, job.j0 + tid / TK, job.k0 + tid % TK, sums);
+    } else {
+        sweep_tile<T, TK, TJ, MODE>(c, job, smem[0], smem[1], acc);
+        if (MODE != MODE_B && !isfinite((acc[2] + acc[4]) + (acc[5] + acc[6]) + acc[7])) {
+            sites_inf<MODE>(args, job.i0, job.i1, job.j0 + tid / TK, job.k0 + tid % TK, sums);
+#pragma unroll
+            for (int q = 0; q < kNV; q++) acc[q] = sums[q];
+        }
+    }
     const int bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
     if constexpr (MODE != MODE_B) {
         block_reduce<kNV>(acc, sred);

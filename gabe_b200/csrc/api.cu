@@ -167,7 +167,8 @@ int fft_r2c(gabe_handle *h, cufftHandle plan, void *in, void *out) {
 
 // The GW chain of step n overlaps the field sweeps of step n+1 (two source
 // buffers) -- except with the library's FFT, which runs in line (measured
-// faster at 512^3) and uses the second buffer as its column passes' target.
+// faster at 512^3; the in-layout and transposed ones use the second buffer
+// as a pass's target).
 bool overlapped(const gabe_handle *h) { return h->evolve_gw && h->S2 && !h->own_fft && !h->fftt && !h->fftp; }
 float *fft_scratch(const gabe_handle *h) { return h->own_fft ? static_cast<float *>(h->S2) : nullptr; }
 void *source_buffer(const gabe_handle *h, int slot) { return slot && h->S2 ? h->S2 : h->S; }
@@ -183,12 +184,10 @@ int source_fft(gabe_handle *h, int slot, cudaStream_t s) {
         CK(h, fftt_cols_f32(h->N, h->S2, S, 2 * kSrc, &h->sc->status, s));
         return GABE_OK;
     }
-    if (h->fftp) {  // the planes of the stage-0 and of the stage-1 sources, S -> S2; the lines run in the k-space update
-        const int n = kSrc * h->N;
-        const size_t in = (size_t)n * h->N * h->N, out = (size_t)n * h->N * (h->N + 2);  // floats of one stage
+    if (h->fftp) {  // the planes of the stage-0 and of the stage-1 sources; the lines run in the k-space update
+        const size_t stage = (size_t)kSrc * h->N * h->N * (h->N + 2);  // floats
         for (int st = 0; st < 2; st++)
-            CK(h, fftp_planes_f32(h->N, static_cast<const float *>(S) + st * in, static_cast<float *>(h->S2) + st * out,
-                                  n, s));
+            CK(h, fftp_planes_f32(h->N, static_cast<float *>(S) + st * stage, kSrc * h->N, s));
         return GABE_OK;
     }
     if (h->own_fft) {
@@ -208,7 +207,7 @@ int kspace(gabe_handle *h, int slot, cudaStream_t s) {
     k.c = h->lc;
     k.slot = slot;
     if (h->fftp) {
-        CK(h, fftp_lines_f32(h->N, h->S2, h->G, h->sc, nullptr, 1, h->lc, slot, s));
+        CK(h, fftp_lines_f32(h->N, h->S, h->G, h->sc, nullptr, 1, h->lc, slot, s));
         return GABE_OK;
     }
     if (h->fftt) {
@@ -228,7 +227,7 @@ StencilArgs stencil_args(gabe_handle *h, int cur, int slot = 0) {
     a.Do = h->D[1 - cur];
     a.S = source_buffer(h, slot);
     a.slot = slot;
-    a.tight = h->fftt || h->fftp;
+    a.src = h->fftp ? SRC_PLANES : h->fftt ? SRC_ROWS : SRC_PADDED;
     a.partials = h->partials;
     a.sc = h->sc;
     a.c = h->lc;
@@ -539,13 +538,7 @@ int gabe_create(const gabe_params *p, gabe_handle **out) {
     if ((rc = dalloc(h, &h->S, h->S_bytes))) return bail(rc);
     if (h->fftt) {  // the transposed transform's first pass writes out of place
         if ((rc = dalloc(h, &h->S2, h->S_bytes))) return bail(rc);
-    } else if (h->fftp) {  // so does the plane pass; without the memory, cuFFT's plan in place
-        if (dalloc(h, &h->S2, h->S_bytes) != GABE_OK) {
-            h->S2 = nullptr;
-            h->fftp = false;
-            h->err.clear();
-        }
-    } else if (h->evolve_gw && !(p->flags & GABE_FLAG_NO_OVERLAP)) {
+    } else if (h->evolve_gw && !h->fftp && !(p->flags & GABE_FLAG_NO_OVERLAP)) {
         // optional: without it the GW chain simply runs in line
         if (dalloc(h, &h->S2, h->S_bytes) != GABE_OK) {
             h->S2 = nullptr;
@@ -723,20 +716,19 @@ static int profile_fftt_passes(gabe_handle *h, int nreps, double ms_out[3]) {
         rc = sweep(h, MODE_A_GW, c, 0, 0);
         if (rc) break;
         cudaError_t ce = cudaEventRecord(e[0], h->stream);
-        const float *S = static_cast<const float *>(h->S);
-        float *S2 = static_cast<float *>(h->S2);
-        const size_t in = (size_t)kSrc * h->N * h->N * h->N, out = in + (size_t)kSrc * h->N * h->N * 2;
+        float *S = static_cast<float *>(h->S);
+        const size_t stage = (size_t)kSrc * h->N * h->N * (h->N + 2);
         unsigned int *st = &h->sc->status;
         if (ce == cudaSuccess)
-            ce = h->fftp ? fftp_planes_f32(h->N, S, S2, kSrc * h->N, h->stream)
-                         : fftt_rows_f32(h->N, S, S2, 2 * kSrc, st, h->stream);
+            ce = h->fftp ? fftp_planes_f32(h->N, S, kSrc * h->N, h->stream)
+                         : fftt_rows_f32(h->N, S, h->S2, 2 * kSrc, st, h->stream);
         if (ce == cudaSuccess) ce = cudaEventRecord(e[1], h->stream);
         if (ce == cudaSuccess)
-            ce = h->fftp ? fftp_planes_f32(h->N, S + in, S2 + out, kSrc * h->N, h->stream)
+            ce = h->fftp ? fftp_planes_f32(h->N, S + stage, kSrc * h->N, h->stream)
                          : fftt_cols_f32(h->N, h->S2, h->S, 2 * kSrc, st, h->stream);
         if (ce == cudaSuccess) ce = cudaEventRecord(e[2], h->stream);
         if (ce == cudaSuccess)
-            ce = h->fftp ? fftp_lines_f32(h->N, h->S2, h->G, h->sc, nullptr, 1, h->lc, 0, h->stream)
+            ce = h->fftp ? fftp_lines_f32(h->N, h->S, h->G, h->sc, nullptr, 1, h->lc, 0, h->stream)
                          : fftt_ikspace_f32(h->N, h->S, h->G, h->sc, h->lc, 0, st, h->stream);
         if (ce == cudaSuccess) ce = cudaEventRecord(e[3], h->stream);
         if (ce != cudaSuccess) {

@@ -26,8 +26,9 @@ using namespace gabe;
 namespace {
 thread_local std::string g_ens_create_error;
 constexpr int kEnsBinBlocks = 32;  // binning blocks per lattice
-// Transformed planes of one batch of the plane transform: the batch size hardly matters (24 to 96 MB 632-637 ms
-// per 50 steps of the 256-lattice ensemble, 1 GB 639), so it is kept small; one stream instead of two 672.
+// Sources of one batch of the plane transform: batches on two streams let the lines of one run beside the planes of
+// another (256-lattice ensemble, 50 steps: one stream instead of two 672 ms against 632).  Their size hardly matters
+// (24 to 96 MB 632-637 ms, 1 GB 639).
 constexpr size_t kPlaneBatchBytes = (size_t)48 << 20;
 }  // namespace
 
@@ -59,10 +60,9 @@ struct gabe_ensemble {
     unsigned int *d_lat_count = nullptr;
     DevScalars *d_sc = nullptr;
     int nkchunks = 0;
-    // the plane transform's batches alternate between two side streams, each with the transformed planes of one
+    // the plane transform's batches alternate between two side streams
     cudaStream_t side[2] = {nullptr, nullptr};
     cudaEvent_t ev_a = nullptr, ev_side[2] = {nullptr, nullptr};
-    float *T[2] = {nullptr, nullptr};
     int gw_launches = 0; // plane transform and k-space launches per step
     void *fft_work = nullptr;
     double *d_m2 = nullptr, *d_sumsq = nullptr;
@@ -219,7 +219,7 @@ int enqueue_step(gabe_ensemble *e, int cur) {
     if (e->gws) {
         // The GW chain reads what sweep A wrote (sources, DevScalars::gw) and nothing that sweep B writes: its
         // batches run on the side streams beside sweep B, filling each other's last waves.
-        if (e->T[0]) {
+        if (e->side[0]) {
             ECK(e, cudaEventRecord(e->ev_a, e->stream));
             for (int b = 0; b < 2; b++) ECK(e, cudaStreamWaitEvent(e->side[b], e->ev_a, 0));
         }
@@ -233,8 +233,8 @@ int enqueue_step(gabe_ensemble *e, int cur) {
             const size_t slots = (size_t)2 * kSrc * G.N * G.N * (G.N + 2), M4 = 4 * lattice_M(G.N);
             for (int l0 = 0; l0 < ng; l0 += G.batch, turn ^= 1) {
                 const int n = std::min(G.batch, ng - l0);
-                ECK(e, fftp_planes_f32(G.N, G.S + l0 * slots, e->T[turn], n * 2 * kSrc * G.N, e->side[turn]));
-                ECK(e, fftp_lines_f32(G.N, e->T[turn], G.G + l0 * M4, e->d_sc, G.ids + l0, n, e->h_lat[G.lats[0]].c, 0,
+                ECK(e, fftp_planes_f32(G.N, G.S + l0 * slots, n * 2 * kSrc * G.N, e->side[turn]));
+                ECK(e, fftp_lines_f32(G.N, G.S + l0 * slots, G.G + l0 * M4, e->d_sc, G.ids + l0, n, e->h_lat[G.lats[0]].c, 0,
                                       e->side[turn]));
             }
         }
@@ -245,7 +245,7 @@ int enqueue_step(gabe_ensemble *e, int cur) {
     }
     int rc2 = sweep(e, MODE_B, cur);
     if (rc2) return rc2;
-    if (e->gws && e->T[0])
+    if (e->gws && e->side[0])
         for (int b = 0; b < 2; b++) {
             ECK(e, cudaEventRecord(e->ev_side[b], e->side[b]));
             ECK(e, cudaStreamWaitEvent(e->stream, e->ev_side[b], 0));
@@ -334,15 +334,13 @@ int gabe_ensemble_create(const gabe_ensemble_params *p, gabe_ensemble **out) {
     }
     int rc;
     if (e->gws) {
-        // batches of the plane transform: the transformed planes of one (10 N^2 (N+2) floats per lattice) fit
-        // the L2 cache beside the sources streaming through it
-        size_t tmax = 0;
+        bool planes = false;
         for (auto &G : e->groups) {
             G.plane = fftp_supported(G.N);
             if (!G.plane) continue;
             const size_t one = (size_t)2 * kSrc * G.N * G.N * (G.N + 2) * sizeof(float);
             G.batch = std::max<int>(1, (int)std::min<size_t>(G.lats.size(), kPlaneBatchBytes / one));
-            tmax = std::max(tmax, G.batch * one);
+            planes = true;
             e->gw_launches += 2 * (int)((G.lats.size() + G.batch - 1) / G.batch);
             if ((rc = ealloc(e, (void **)&G.ids, sizeof(int) * G.lats.size()))) return bail(rc);
             if (cudaMemcpy(G.ids, G.lats.data(), sizeof(int) * G.lats.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
@@ -351,8 +349,7 @@ int gabe_ensemble_create(const gabe_ensemble_params *p, gabe_ensemble **out) {
                 return bail(GABE_ERR_CUDA);
             }
         }
-        for (int b = 0; tmax && b < 2; b++) {
-            if ((rc = ealloc(e, (void **)&e->T[b], tmax))) return bail(rc);
+        for (int b = 0; planes && b < 2; b++) {
             if (cudaStreamCreateWithFlags(&e->side[b], cudaStreamNonBlocking) != cudaSuccess ||
                 cudaEventCreateWithFlags(&e->ev_side[b], cudaEventDisableTiming) != cudaSuccess ||
                 (b == 0 && cudaEventCreateWithFlags(&e->ev_a, cudaEventDisableTiming) != cudaSuccess)) {

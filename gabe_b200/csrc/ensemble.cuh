@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(kEnsThreads, s32::sweep32_threads_per_sm<MODE>
     t.i0 = item.i0;
     t.i1 = item.i1;
     t.planes = 0;
-    t.tight = L.gt == 2;  // the plane transform
+    t.src = L.gt == 2 ? SRC_PLANES : SRC_PADDED;
     __shared__ s32::Site32 s;
     // by a warp that copies nothing; the march waits for the block before it reads them
     if (tid == (int)blockDim.x - 1) s32::site32_consts<MODE>(c, L.sc, s);

@@ -21,14 +21,14 @@ cudaError_t grid_of(K kernel, int threads, size_t smem, int ntiles, int *grid) {
 }
 
 template <int N>
-cudaError_t planes_n(const float *S, float2 *T, int nplanes, cudaStream_t s) {
+cudaError_t planes_n(float *S, int nplanes, cudaStream_t s) {
     constexpr size_t smem = f2p::PlaneGeom<N>::SMEM_BYTES;
     auto k = f2p::plane_kernel<N>;
     const int ntiles = nplanes / f2p::Cfg<N>::PB;
     int g = 0;
     cudaError_t e = grid_of(k, f2p::Cfg<N>::TP, smem, ntiles, &g);
     if (e != cudaSuccess) return e;
-    k<<<g, f2p::Cfg<N>::TP, smem, s>>>(S, T, ntiles);
+    k<<<g, f2p::Cfg<N>::TP, smem, s>>>(S, ntiles);
     return cudaGetLastError();
 }
 
@@ -53,10 +53,10 @@ bool fftp_supported(int N) {
 #undef X
 }
 
-cudaError_t fftp_planes_f32(int N, const float *S, void *T, int nplanes, cudaStream_t s) {
+cudaError_t fftp_planes_f32(int N, float *S, int nplanes, cudaStream_t s) {
     switch (N) {
 #define X(n) \
-    case n: return planes_n<n>(S, static_cast<float2 *>(T), nplanes, s);
+    case n: return planes_n<n>(S, nplanes, s);
         GABE_F2P_SIZES(X)
 #undef X
         default: return cudaErrorInvalidValue;

@@ -6,11 +6,12 @@
 // (fft_stresstensor, g2evolutionpert.cpp:183-195) and then updates h and l
 // per k-point (evolve_perts, :343-455).
 //
-//   plane pass  (plane_kernel)  S[q][i][j][N+2] -> T[q][i][x]
+//   plane pass  (plane_kernel)  S[q][i][j][k] -> T[q][i][x], in place
 //       rows along k (two real rows as one complex sequence), then columns
 //       along j of a whole (j, k) plane in shared memory, both as four-step
 //       FFTs N = L1 L2; the plane's half spectrum has the flat index
-//       x = ky (N/2+1) + kz;
+//       x = ky (N/2+1) + kz and takes the N (N + 2) reals that the plane's
+//       N rows of N begin (SRC_PLANES);
 //   lines pass  (lines_kernel)  T, G[p][x / 8][kx][x % 8]
 //       takes the lines along i of eight neighbouring x (64-byte pieces) of
 //       the ten arrays: it transforms the 80 lines, and each k-point's update
@@ -127,10 +128,11 @@ __device__ __forceinline__ int place(int e) {
 
 template <int N>
 __global__ void __launch_bounds__(Cfg<N>::TP, Cfg<N>::MBP)
-    plane_kernel(const float *__restrict__ S, float2 *__restrict__ T, int ntiles) {
+    plane_kernel(float *S, int ntiles) {
     using G = PlaneGeom<N>;
     using C = Cfg<N>;
     constexpr int L1 = C::L1, L2 = C::L2, NH = G::NH, RP = G::RP, PR = G::PR, TP = C::TP, PB = C::PB;
+    constexpr int PP = N * (N + 2);  // reals from plane to plane
     extern __shared__ __align__(128) unsigned char sm[];
     float2 *tw = reinterpret_cast<float2 *>(sm);
     float *W = reinterpret_cast<float *>(sm + N * sizeof(float2));
@@ -140,11 +142,10 @@ __global__ void __launch_bounds__(Cfg<N>::TP, Cfg<N>::MBP)
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         // rows, first step: L2-point DFTs over n2 (stride L1) of two neighbouring n1, twiddled,
         // from global memory to element k2 + L2 n1 of the work layout
-        // (the sources of one lattice after another stand 2 kSrc N^2 (N + 2) floats apart)
-        const float *src = S + (size_t)tile * G::ROWS * RP + (size_t)(tile / (2 * kSrc * N / PB)) * (2 * kSrc * N * N * 2);
+        float *src = S + (size_t)tile * (PB * PP);
         for (int t = tid; t < G::PAIRS * (L1 / 2); t += TP) {
             const int p = t / (L1 / 2), n1 = 2 * (t % (L1 / 2));
-            const float *re = src + 2 * p * RP + n1, *im = re + RP;
+            const float *re = src + (2 * p / N) * PP + (2 * p % N) * RP + n1, *im = re + RP;
             float2 xa[L2], xb[L2];
 #pragma unroll
             for (int n2 = 0; n2 < L2; n2++) {
@@ -224,11 +225,9 @@ __global__ void __launch_bounds__(Cfg<N>::TP, Cfg<N>::MBP)
             put(xb, n1 + 1, row + PR);
         }
         __syncthreads();
-        // columns, second step, to HBM: ky = k2 + L2 k1, x = ky NH + kz
+        // columns, second step, over the planes: ky = k2 + L2 k1, x = ky NH + kz
         {
-            const int plane0 = tile * PB;
-            const int q = plane0 / N, i0 = plane0 % N;
-            float2 *To = T + (size_t)q * ((size_t)N * N * NH) + (size_t)i0 * (N * NH);
+            float2 *To = reinterpret_cast<float2 *>(src);  // every read of the tile's rows lies behind three barriers
             for (int t = tid; t < PB * NH * L2; t += TP) {
                 const int kz = t % NH, m = t / NH, k2 = m % L2, b = m / L2;
                 const int re = place<N>(kz), im = place<N>(im_at<N>(kz));

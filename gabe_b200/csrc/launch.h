@@ -213,12 +213,12 @@ cudaError_t fftt_cols_f32(int N, const void *T1, void *T2, int ncomp, unsigned i
 cudaError_t fftt_ikspace_f32(int N, const void *T2, void *G, const DevScalars *sc, const LatticeConsts &c, int slot,
                              unsigned int *status, cudaStream_t s);
 
-// FP32 plane transform (fftp.cuh), N a multiple of 16 up to 160: the (j, k) planes of nplanes
-// consecutive planes S[..][N][N+2] -> T[..][x], x = ky (N/2+1) + kz (nplanes = N per source array), and the
-// lines along i of nlat lattices of ten arrays each fused with the TT projection and h/l update of
-// their amplitudes G (order of g_index, gt = 2); lattice l's scalars are sc[ids ? ids[l] : l].
+// FP32 plane transform (fftp.cuh), N a multiple of 16 up to 160: nplanes consecutive (j, k) planes S (SRC_PLANES:
+// N rows of N reals, N (N + 2) reals apart; nplanes = N per source array) -> T[..][x], x = ky (N/2+1) + kz, in place,
+// and the lines along i of nlat lattices of ten arrays T each fused with the TT projection and h/l update of their
+// amplitudes G (order of g_index, gt = 2); lattice l's scalars are sc[ids ? ids[l] : l].
 bool fftp_supported(int N);
-cudaError_t fftp_planes_f32(int N, const float *S, void *T, int nplanes, cudaStream_t s);
+cudaError_t fftp_planes_f32(int N, float *S, int nplanes, cudaStream_t s);
 cudaError_t fftp_lines_f32(int N, const void *T, void *G, const DevScalars *sc, const int *ids, int nlat,
                            const LatticeConsts &c, int slot, cudaStream_t s);
 

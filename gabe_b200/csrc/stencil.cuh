@@ -40,6 +40,13 @@ namespace gabe {
 
 enum SweepMode : int { MODE_A = 0, MODE_A_GW = 1, MODE_E0 = 2, MODE_B = 3 };
 
+// FP32 GW sources [10][i][j][k]: rows of N + 2 reals for a transform that takes each row in place, rows of N for the
+// library's transposed and plane transforms.  A warp's store is then two whole 128-byte lines instead of parts of
+// three: sweep A at 512^3 1.39 ms against 1.70, at 128^3 37.4 us against 40.6; the plane pass at 128^3 64.7 us against
+// 69.4, the transposed rows unchanged.  The plane transform writes a (j, k) plane's half spectrum over the plane, so
+// its planes of N rows stand N (N + 2) reals apart.
+enum SrcLayout { SRC_PADDED = 0, SRC_ROWS = 1, SRC_PLANES = 2 };
+
 struct StencilArgs {
     const void *X;       // fields in  [2][N^3]
     const void *D;       // momenta in [2][N^3]
@@ -63,11 +70,7 @@ struct StencilArgs {
     // Host memory (mapped) that receives the scalars after the last block has
     // finished the stage, or null: a caller that waits for them saves the copy.
     DevScalars *mirror;
-    // FP32 sources in rows of N reals instead of N + 2, for the transforms that work out of place (the plane and
-    // the transposed one; an in-place r2c needs the padding): each warp store is then two whole 128-byte lines
-    // instead of parts of three.  Sweep A at 512^3 1.39 ms against 1.70, at 128^3 37.4 us against 40.6; the plane
-    // pass at 128^3 64.7 us against 69.4, the transposed rows unchanged.
-    bool tight;
+    SrcLayout src;  // layout of the FP32 sources
 };
 
 constexpr int kNV = 8;  // reduced values: kin0 pot0 grad0 | pot1 grad1 PP PQ QQ

@@ -201,8 +201,8 @@ constexpr int sweep32_threads_per_sm() {
 struct Tile32 {
     const float *X, *D;  // fields and momenta of the current state, [2][N^3]
     float *Xo, *Do;      // new fields and momenta (sweep B)
-    float *S;            // GW sources [10][N][N][row] (sweep A with sources; a slab: its own planes)
-    bool tight;          // row = N instead of N + 2: a warp's stores are then whole 128-byte lines
+    float *S;            // GW sources (sweep A with sources; a slab: its own planes)
+    SrcLayout src;       // ... in this layout
     int k0, j0, i0, i1;
     int planes;          // planes per field in X, D, Xo, Do (slab, no wrap along i); 0 = N, periodic
 };
@@ -265,9 +265,10 @@ __device__ __forceinline__ void march32(const LatticeConsts &c, const Site32 &s,
         if (p <= i1) issue(p, q);
         cp_commit();
     }
-    // sources [10][planes][N][row]: the whole lattice, or a slab's own planes (plane i at i - 1)
+    // sources of the whole lattice, or of a slab's own planes (plane i at i - 1)
     const int splanes = t.planes ? t.planes - 2 : N, sfirst = t.planes ? 1 : 0;
-    const int srow = t.tight ? N : N + 2, sstride = splanes * N * srow;  // one source component
+    const int srow = t.src == SRC_PADDED ? N + 2 : N, splane = N * (t.src == SRC_ROWS ? N : N + 2);
+    const int sstride = splanes * splane;  // one source component
     const int so_row = j * srow + k;
     using Own = F2[4];  // the own pair of the four arrays in one plane
     auto own = [&](int sl, int a) {
@@ -310,7 +311,7 @@ __device__ __forceinline__ void march32(const LatticeConsts &c, const Site32 &s,
                     ngroup = 0;
                 }
                 if constexpr (MODE == MODE_A_GW) {
-                    float *g = t.S + ((i - sfirst) * (N * srow) + so_row);
+                    float *g = t.S + ((i - sfirst) * splane + so_row);
 #pragma unroll
                     for (int q = 0; q < kSrc; q++, g += sstride) __stcs(reinterpret_cast<float2 *>(g), unpack(s0[q]));
 #pragma unroll
@@ -356,7 +357,7 @@ __global__ void __launch_bounds__(TK2 *TJ, (sweep32_threads_per_sm<MODE>() + TK2
     t.k0 = blockIdx.x * 2 * TK2;
     t.j0 = blockIdx.y * TJ;
     t.planes = args.planes;
-    t.tight = args.tight;
+    t.src = args.src;
     const int first = args.planes ? 1 : 0, end = args.planes ? args.planes - 1 : N;  // own planes
     t.i0 = first + blockIdx.z * args.ci;
     t.i1 = min(t.i0 + args.ci, end);

@@ -72,7 +72,8 @@ enum gabe_flags {
                                  words of device memory).  With the library's 3-D FFT the chain runs
                                  in line anyway and the second buffer is the target of its column
                                  passes (out of place, faster); this flag makes them in place.  The
-                                 transposed and plane transforms need the second buffer in any case */
+                                 transposed transform needs the second buffer in any case, the plane
+                                 transform never does */
     GABE_FLAG_OWN_FFT = 16,     /* FP32 with N in {64, 128, 256, 512}: transform the GW sources with the
                                    library's in-layout three-pass 3-D r2c (the layout of a library r2c)
                                    followed by the separate k-space pass, instead of the default */

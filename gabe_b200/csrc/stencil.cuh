@@ -576,17 +576,15 @@ __global__ void __launch_bounds__(TK *TJ) sweep_kernel(const __grid_constant__ S
     const int tid = threadIdx.x;
     static_assert(sizeof(smem) >= TK * TJ * kNV * sizeof(double), "the tile buffers hold the sums of sites_inf");
     double *sums = &smem[0][0] + tid * kNV;
-    // Infinite quotients make the state's energies infinite or NaN.  Sweep B knows that from sweep A; sweep A and the
-    // energies see it in their own sums.
-    if (MODE == MODE_B && (args.sc->status & ST_NONFINITE)) {
+    // Infinite quotients make the state's energies infinite or NaN.  Sweep A and the energies see it in their own sums,
+    // sweep B in the status that sweep A left (read before the march, whose loads need not wait for it).
+    const unsigned int status = MODE == MODE_B ? args.sc->status : 0u;
+    sweep_tile<T, TK, TJ, MODE>(c, job, smem[0], smem[1], acc);
+    if (MODE == MODE_B ? (status & ST_NONFINITE) != 0 : !isfinite((acc[2] + acc[4]) + (acc[5] + acc[6]) + acc[7])) {
         sites_inf<MODE>(args, job.i0, job.i1, job.j0 + tid / TK, job.k0 + tid % TK, sums);
-    } else {
-        sweep_tile<T, TK, TJ, MODE>(c, job, smem[0], smem[1], acc);
-        if (MODE != MODE_B && !isfinite((acc[2] + acc[4]) + (acc[5] + acc[6]) + acc[7])) {
-            sites_inf<MODE>(args, job.i0, job.i1, job.j0 + tid / TK, job.k0 + tid % TK, sums);
+        if constexpr (MODE != MODE_B)
 #pragma unroll
             for (int q = 0; q < kNV; q++) acc[q] = sums[q];
-        }
     }
     const int bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
     if constexpr (MODE != MODE_B) {

@@ -1440,7 +1440,7 @@ struct gabe_mlp {
     float *params = nullptr, *grads = nullptr, *mom = nullptr, *vel = nullptr;
     float *xb = nullptr, *tb = nullptr, *y = nullptr, *dy = nullptr, *d0 = nullptr, *d1 = nullptr;
     float *ws = nullptr, *dbp = nullptr;  // split-K partials of the weight gradient
-    // batches of at most kSmallRows rows: every layer's gradient of the pre-activations and split-K partials
+    // batches of at most small_rows rows: every layer's gradient of the pre-activations and split-K partials
     float *small_delta = nullptr, *small_ws = nullptr;
     int small_rows = 0;
     std::vector<long long> small_off;  // floats: per layer, weight partials then bias partials
@@ -1490,8 +1490,11 @@ void *act_at(const gabe_mlp *m, void *base, int layer) {
 
 constexpr int kMaxSplits = 16;
 // Batches up to here take the one-launch weight gradients and update, which keep every layer's deltas and
-// partials at once (a bounded buffer); larger ones are long enough per launch.
+// partials at once; larger ones are long enough per launch.  So are those of wide networks: the two buffers take
+// no more than kSmallBytes (the default network's 34 MB), with fewer rows or none, and a handle does without them
+// where the memory is not there.
 constexpr int kSmallRows = 4096;
+constexpr long long kSmallBytes = 256ll << 20;
 
 // Splits of the batch for the weight gradient of a K x N layer, enough for about two blocks per SM, and the
 // rows of one split.
@@ -1987,7 +1990,6 @@ int gabe_mlp_create(const gabe_mlp_params *p, gabe_mlp **out) {
     }
     const size_t R = p->max_rows, W = p->width, A = act_size(m);
     const size_t wide = (size_t)(p->n_out > p->width ? p->n_out : p->width);
-    m->small_rows = p->max_rows < kSmallRows ? p->max_rows : kSmallRows;
     long long small_ws = 0;
     for (int l = 0; l < m->nl; l++) {
         const long long splits = most_splits(m->K[l], m->N[l]);
@@ -2007,13 +2009,25 @@ int gabe_mlp_create(const gabe_mlp_params *p, gabe_mlp **out) {
         {(void **)&m->part, kLossBlocks * sizeof(double2)}, {(void **)&m->ts, sizeof(TrainScalars)},
         {(void **)&m->ws, (size_t)kMaxSplits * wide * wide * 4}, {(void **)&m->dbp, (size_t)kMaxSplits * wide * 4},
         {(void **)&m->wt, (size_t)(nwt > 0 ? nwt : 1) * sizeof(bf16)}, {(void **)&m->status, sizeof(unsigned int)},
-        {(void **)&m->small_delta, (size_t)p->depth * m->small_rows * W * 4}, {(void **)&m->small_ws, (size_t)small_ws * 4},
     };
     for (auto &a : allocs) {
         if (cudaMalloc(a.ptr, a.bytes) != cudaSuccess) {
             cudaGetLastError();
             mset(m, GABE_ERR_NOMEM, "cudaMalloc(%zu bytes) failed", a.bytes);
             return fail(GABE_ERR_NOMEM);
+        }
+    }
+    const long long row_bytes = (long long)p->depth * p->width * 4, fit = (kSmallBytes - small_ws * 4) / row_bytes;
+    long long small_rows = p->max_rows < kSmallRows ? p->max_rows : kSmallRows;
+    if (small_rows > fit) small_rows = fit;
+    if (small_rows > 0) {
+        if (cudaMalloc((void **)&m->small_delta, (size_t)(small_rows * row_bytes)) == cudaSuccess &&
+            cudaMalloc((void **)&m->small_ws, (size_t)small_ws * 4) == cudaSuccess) {
+            m->small_rows = (int)small_rows;
+        } else {  // every batch takes the kernels of the large ones
+            cudaGetLastError();
+            if (m->small_delta) cudaFree(m->small_delta);
+            m->small_delta = m->small_ws = nullptr;
         }
     }
     // Glorot-uniform weights, zero biases, from the seed

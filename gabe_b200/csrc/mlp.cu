@@ -1443,6 +1443,7 @@ struct gabe_mlp {
     // batches of at most small_rows rows: every layer's gradient of the pre-activations and split-K partials
     float *small_delta = nullptr, *small_ws = nullptr;
     int small_rows = 0;
+    int batch = 1;  // of the last gabe_mlp_train call
     std::vector<long long> small_off;  // floats: per layer, weight partials then bias partials
     bf16 *wt = nullptr;              // BF16 transposed weights of layers >= 1 (tensor-core forward)
     tc::WtTable wtab{};
@@ -2128,6 +2129,7 @@ int gabe_mlp_loss_grad(gabe_mlp *m, const float *x, const float *t, int64_t n, d
 int gabe_mlp_train(gabe_mlp *m, const float *x, const float *t, const int32_t *perm, int32_t batch, int32_t nbatch) {
     if (!m || !x || !t || !perm || batch < 1 || batch > m->p.max_rows || nbatch < 0) return GABE_ERR_PARAM;
     MCK(m, cudaSetDevice(m->dev));
+    m->batch = batch;
     if (!(m->p.flags & GABE_MLP_NO_GRAPH) &&
         (!m->gexec || m->g_x != x || m->g_t != t || m->g_perm != perm || m->g_batch != batch)) {
         if (m->gexec) cudaGraphExecDestroy(m->gexec);
@@ -2215,8 +2217,10 @@ int gabe_mlp_forward_form(const gabe_mlp *m, int32_t layer) {
 void *gabe_mlp_stream(const gabe_mlp *m) { return m ? (void *)m->stream : nullptr; }
 
 int gabe_mlp_launches_per_train_step(const gabe_mlp *m) {
-    // batches of at most kSmallRows: gather, forward, loss, data gradients, weight gradients, update
-    return m ? 2 + (m->fused_slots ? 1 : m->nl) + (m->nl - 1) + 2 : 0;
+    if (!m) return 0;
+    const int n = 2 + (m->fused_slots ? 1 : m->nl) + (m->nl - 1);  // gather, forward, loss, data gradients
+    if (m->batch <= m->small_rows) return n + 2;                   // weight gradients, update
+    return n + 2 * m->nl + 1 + (m->f32act ? 0 : 1);                // ... and reductions, update, BF16 weights
 }
 
 

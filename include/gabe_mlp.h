@@ -94,7 +94,9 @@ int gabe_mlp_sync(gabe_mlp *m);
  * 2 tcgen05; -1 for a bad layer index. */
 int gabe_mlp_forward_form(const gabe_mlp *m, int32_t layer);
 void *gabe_mlp_stream(const gabe_mlp *m);
-/* The library's kernel launches per training step and per forward chunk. */
+/* The library's kernel launches per training step (of the last gabe_mlp_train
+ * call's batch; before any, of a single row: batches of up to 4096 rows, fewer
+ * in wide networks, take fewer launches) and per forward chunk. */
 int gabe_mlp_launches_per_train_step(const gabe_mlp *m);
 int gabe_mlp_launches_per_forward(const gabe_mlp *m);
 const char *gabe_mlp_last_error(const gabe_mlp *m);

@@ -29,6 +29,9 @@ SHAPES32 = {0: (64, 8), 1: (64, 4), 2: (128, 4), 3: (32, 8), 4: (64, 16), 5: (32
 
 def shapes_for(precision: int) -> dict:
     return SHAPES32 if precision == FP32 else SHAPES
+
+
+FINAL_ROUNDS = 5  # timings of each tile among the fastest
 CACHE = os.environ.get("GABE_TILE_CACHE", os.path.join(os.path.dirname(os.path.abspath(__file__)), "tiles.json"))
 
 
@@ -111,21 +114,25 @@ def candidates(N: int, precision: int = FP32):
     for s, (tk, tj) in shapes_for(precision).items():
         if tk > N or tj > N or N % tk or N % tj:
             continue
-        for ci in (16, 32, 64, 128, 256, 512):
+        for ci in (4, 8, 16, 32, 64, 128, 256, 512):
             if ci <= N:
                 out.append((s, ci))
     return out
 
 
 def tune(N: int, precision: int = FP32, gws: bool = True, steps: int = 3, verbose: bool = True) -> dict:
-    """Times every candidate on a random state; returns and caches the best."""
+    """Times every candidate on a random state, then those within 5 % of the
+    best FINAL_ROUNDS times more in turn (tiles that close change places with
+    the clock from one timing to the next); returns and caches the one with
+    the shortest median -- among tiles within 1 % of that, the first of the
+    table, which is the one that plan_grid32 takes by itself where it can."""
     rng = np.random.default_rng(0)
     f = 0.342 + 1e-6 * rng.standard_normal((2, N, N, N))
     f[1] -= 0.342
     d = 1e-6 * rng.standard_normal((2, N, N, N))
-    results = []
     table = shapes_for(precision)
-    for shape, ci in candidates(N, precision):
+
+    def once(shape, ci):
         try:
             with Lattice(N, gws=gws, precision=precision, tile_shape=shape, tile_ci=ci) as lat:
                 lat.upload_state(f, d, a0=1.0, adot0=0.5)
@@ -134,13 +141,25 @@ def tune(N: int, precision: int = FP32, gws: bool = True, steps: int = 3, verbos
         except GabeError as e:
             if verbose:
                 print(f"shape {table[shape]} ci {ci}: {e}")
-            continue
-        t = ph["stage1"] + ph["stage2"]
-        results.append({"shape": shape, "ci": ci, "sweeps_ms": t, "stage1": ph["stage1"], "stage2": ph["stage2"]})
+            return None
         if verbose:
-            print(f"shape {table[shape]} ci {ci:4d}: sweep A {ph['stage1']:.3f} ms  sweep B {ph['stage2']:.3f} ms",
+            print(f"shape {table[shape]} ci {ci:4d}: sweep A {ph['stage1']:.4f} ms  sweep B {ph['stage2']:.4f} ms",
                   flush=True)
-    best = min(results, key=lambda r: r["sweeps_ms"])
+        return {"shape": shape, "ci": ci, "sweeps_ms": ph["stage1"] + ph["stage2"], "stage1": ph["stage1"],
+                "stage2": ph["stage2"]}
+
+    results = [r for r in (once(s, ci) for s, ci in candidates(N, precision)) if r]
+    fastest = min(r["sweeps_ms"] for r in results)
+    close = [(r["shape"], r["ci"]) for r in results if r["sweeps_ms"] <= 1.05 * fastest]
+    final = {c: [] for c in close}
+    for _ in range(FINAL_ROUNDS if len(close) > 1 else 0):
+        for c in close:
+            r = once(*c)
+            if r:
+                final[c].append(r)
+    finals = [sorted(v, key=lambda r: r["sweeps_ms"])[len(v) // 2] for v in final.values() if v] or results
+    shortest = min(r["sweeps_ms"] for r in finals)
+    best = next(r for r in finals if r["sweeps_ms"] <= 1.01 * shortest)
     cache = load_cache()
     cache[_key(N, precision, gws)] = {"shape": best["shape"], "ci": best["ci"], "sweeps_ms": best["sweeps_ms"],
                                       "tile": table[best["shape"]]}

@@ -107,9 +107,10 @@ inline GridPlan plan_grid32(int N, int want_shape, int want_ci) {
     if (shape < 0) return GridPlan{-1, 0, dim3(0, 0, 0)};  // no tile divides N (N % 16 != 0)
     const int TK = kShapes32[shape][0], TJ = kShapes32[shape][1];
     const int bxy = (N / TK) * (N / TJ);
-    // planes per block: N / 8 from N = 128 on (the fastest measured at 128^3, 256^3 and 512^3, where 64 x 8
-    // columns of 64 planes take 2.23 ms for both sweeps, 128 x 4 2.30, 32 planes 2.32); below, enough blocks for four
-    // per SM
+    // planes per block: N / 8 from N = 128 on, within 1 % of the fastest of all shapes and plane counts at 128^3,
+    // 256^3 and 512^3 with GWs (both sweeps 62.1 us; 0.296 ms, 64 x 4 columns 0.297; 2.18 ms, 64 x 8 of 32 or 256
+    // planes 2.24, 128 x 4 of 64 2.20); below, enough blocks for four per SM (64^3: 64 x 8 of 4 planes 28.2 us, 64 x 4
+    // of 4 or 8 29)
     int ci = want_ci > 0 ? want_ci : (N >= 128 ? N / 8 : N);
     if (want_ci <= 0 && N < 128)
         while (ci > 4 && (long long)bxy * ((N + ci - 1) / ci) < 4 * 148) ci /= 2;

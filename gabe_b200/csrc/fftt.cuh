@@ -8,9 +8,9 @@
 // lines of its own axis as contiguous runs and writes its output transposed,
 // so that the next pass's lines are contiguous again:
 //
-//   pass 1 (rowt_kernel)   S[q][i][j][N+2] reals   -> T1[q][i][kz][j]
+//   pass 1 (rowt_kernel)   S[q][i][j][k] reals, rows of N (SRC_ROWS)  -> T1[q][i][kz][j]
 //          rows along k, two real rows as one complex sequence, 16-row
-//          tiles landed by one bulk copy each, each kz written as one
+//          tiles landed by bulk copies, each kz written as one
 //          128-byte piece of 16 consecutive j (eight 16-byte pair stores);
 //   pass 2 (colt_kernel)   T1 lines along j         -> T2[q][kz][ky][i]
 //          16 lines of consecutive i per tile, landed in shared memory by
@@ -44,10 +44,10 @@ using pfft::FourStep;
 // ---------------------------------------------------------------------------
 // A tile of 16 rows (8 pairs, each two real rows taken as one complex
 // sequence) is one contiguous run of S and lands in shared memory by one bulk
-// copy (cp.async.bulk + mbarrier); for N < 512 by one per row, N + L1 / 2
-// floats apart, so that the pairs that half a warp reads together start on
-// different banks (at 512 it reads of one pair).  The four-step FFT's first pass reads the pairs from
-// the linear buffer (lanes over consecutive elements: conflict-free) and
+// copy (cp.async.bulk + mbarrier; one per row, padded so that the pairs which
+// half a warp reads together start on different banks, ran 330 us against 301
+// at 256^3, 43.6 against 42.0 at 128^3).  The four-step FFT's first pass reads
+// the pairs from the linear buffer (lanes over consecutive elements) and
 // writes its output into a work buffer in the pair-preserving XOR swizzle of
 // fft3d.cuh, so that the second pass's stride-L1 reads fall on distinct
 // banks; the linear buffer is refilled as soon as the first pass has read
@@ -70,13 +70,12 @@ using pfft::FourStep;
 template <int N, int T_ = 128, int NB_ = 1>
 struct RowTGeom {
     using RG = f3d::RowGeom<N, 16, 1, T_, 2>;  // the work buffer (swizzled, pitch N + 2)
-    static constexpr int R = 16, RP = RG::L1 == 32 ? N : N + RG::L1 / 2, NB = NB_;
+    static constexpr int R = 16, NB = NB_;
     static constexpr size_t HEAD = 128;                          // NB mbarriers
     static constexpr size_t TW_BYTES = (size_t)N * sizeof(float2);  // twiddles of the four-step
-    static constexpr size_t LIN_BYTES = (size_t)R * RP * sizeof(float);
+    static constexpr size_t LIN_BYTES = (size_t)R * N * sizeof(float);
     static constexpr size_t SMEM_BYTES = HEAD + TW_BYTES + NB * LIN_BYTES + (size_t)RG::BUF * sizeof(float);
     static_assert(LIN_BYTES % 16 == 0 && (HEAD + TW_BYTES) % 16 == 0, "bulk copies of 16-byte multiples");
-    static_assert(RP % 4 == 0, "every row lands on a 16-byte boundary");
 };
 
 template <int N, int T_ = 128, int MINB = 2, int NB_ = 1>
@@ -85,13 +84,13 @@ __global__ void __launch_bounds__(T_, MINB)
     using G = RowTGeom<N, T_, NB_>;
     using Gm = typename G::RG;
     constexpr int L1 = Gm::L1, L2 = Gm::L2, PITCH = Gm::PITCH, R = Gm::R, P = Gm::P, T = Gm::T, NT2 = Gm::NT2;
-    constexpr int RP = G::RP, NB = G::NB, NH = N / 2 + 1;
+    constexpr int NB = G::NB, NH = N / 2 + 1;
     static_assert(R == 16 && P == 8, "one 128-byte output piece per kz");
     extern __shared__ __align__(128) unsigned char sm[];
     uint64_t *bar = reinterpret_cast<uint64_t *>(sm);
     float2 *tw = reinterpret_cast<float2 *>(sm + G::HEAD);
-    float *lin0 = reinterpret_cast<float *>(sm + G::HEAD + G::TW_BYTES);  // [NB][R][RP]
-    float *rows = lin0 + NB * R * RP;                                     // work buffer [R][PITCH], swizzled
+    float *lin0 = reinterpret_cast<float *>(sm + G::HEAD + G::TW_BYTES);  // [NB][R][N]
+    float *rows = lin0 + NB * R * N;                                      // work buffer [R][PITCH], swizzled
     const int tid = threadIdx.x;
     const long long ntiles = nrows / R;
     if (tid == 0) {
@@ -103,11 +102,8 @@ __global__ void __launch_bounds__(T_, MINB)
     int fills[NB] = {};  // thread 0: fills issued per buffer
     auto issue = [&](long long tile, int b) {
         fills[b]++;
-        tma::mbar_arrive_expect(&bar[b], (uint32_t)(R * N * sizeof(float)));
-        const float *src = S + tile * R * N;
-        if constexpr (RP == N) tma::load(lin0 + b * R * RP, src, (uint32_t)G::LIN_BYTES, &bar[b]);
-        else for (int r = 0; r < R; r++)
-            tma::load(lin0 + (b * R + r) * RP, src + r * N, (uint32_t)(N * sizeof(float)), &bar[b]);
+        tma::mbar_arrive_expect(&bar[b], (uint32_t)G::LIN_BYTES);
+        tma::load(lin0 + b * R * N, S + tile * R * N, (uint32_t)G::LIN_BYTES, &bar[b]);
     };
     if (tid == 0)
         for (int q = 0; q < NB; q++) {
@@ -122,12 +118,12 @@ __global__ void __launch_bounds__(T_, MINB)
             if (tid == 0) tma::drain(bar, fills, NB, status);
             break;
         }
-        const float *lin = lin0 + b * R * RP;
+        const float *lin = lin0 + b * R * N;
         // four-step pass 1: L2-point FFTs over n2 (stride L1), twiddle W_N^(n1 k2), in place
         // two adjacent n1 per thread: each pair of reals is one 8-byte access
         for (int t = tid; t < P * (L1 / 2); t += T) {
             const int p = t / (L1 / 2), n1 = 2 * (t % (L1 / 2));
-            const float *lre = lin + 2 * p * RP, *lim = lre + RP;
+            const float *lre = lin + 2 * p * N, *lim = lre + N;
             float *re = rows + 2 * p * PITCH, *im = re + PITCH;
             float2 xa[L2], xb[L2];
 #pragma unroll

@@ -166,10 +166,10 @@ int fft_r2c(gabe_handle *h, cufftHandle plan, void *in, void *out) {
 }
 
 // The GW chain of step n overlaps the field sweeps of step n+1 (two source
-// buffers) -- except with the library's FFT, which runs in line (measured
-// faster at 512^3; the in-layout and transposed ones use the second buffer
-// as a pass's target).
-bool overlapped(const gabe_handle *h) { return h->evolve_gw && h->S2 && !h->own_fft && !h->fftt && !h->fftp; }
+// buffers) -- except with the in-layout and transposed transforms, which run
+// in line (measured faster at 512^3) and use the second buffer as a pass's
+// target.
+bool overlapped(const gabe_handle *h) { return h->evolve_gw && h->S2 && !h->own_fft && !h->fftt; }
 float *fft_scratch(const gabe_handle *h) { return h->own_fft ? static_cast<float *>(h->S2) : nullptr; }
 void *source_buffer(const gabe_handle *h, int slot) { return slot && h->S2 ? h->S2 : h->S; }
 
@@ -207,7 +207,7 @@ int kspace(gabe_handle *h, int slot, cudaStream_t s) {
     k.c = h->lc;
     k.slot = slot;
     if (h->fftp) {
-        CK(h, fftp_lines_f32(h->N, h->S, h->G, h->sc, nullptr, 1, h->lc, slot, s));
+        CK(h, fftp_lines_f32(h->N, k.S, h->G, h->sc, nullptr, 1, h->lc, slot, s));
         return GABE_OK;
     }
     if (h->fftt) {
@@ -528,8 +528,9 @@ int gabe_create(const gabe_params *p, gabe_handle **out) {
     h->fftt = h->evolve_gw && h->f32 && fftt_supported(h->N) &&
               ((p->flags & GABE_FLAG_TRANSPOSED_FFT) ||
                (h->N >= 128 && !(p->flags & (GABE_FLAG_OWN_FFT | GABE_FLAG_CUFFT_3D))));
-    // the plane transform at the sizes it takes except 64 (transform and k-space update at 96^3 61 us against
-    // 108 with cuFFT's plan, at 128^3 114 against 120 with the transposed form), unless a flag names a form
+    // the plane transform at the sizes it takes except 64, unless a flag names a form: a step at 96^3 80 us against
+    // 125 with cuFFT's plan and its chain overlapped, at 128^3 152 against 160 with the transposed form, at 160^3 323
+    // against 425; at 64^3, where every launch is short, 39.0 against 36.9 with cuFFT's overlapped chain
     h->fftp = h->evolve_gw && h->f32 && fftp_supported(h->N) && h->N != 64 &&
               !(p->flags & (GABE_FLAG_OWN_FFT | GABE_FLAG_CUFFT_3D | GABE_FLAG_TRANSPOSED_FFT));
     if (h->fftp) h->fftt = false;
@@ -538,7 +539,10 @@ int gabe_create(const gabe_params *p, gabe_handle **out) {
     if ((rc = dalloc(h, &h->S, h->S_bytes))) return bail(rc);
     if (h->fftt) {  // the transposed transform's first pass writes out of place
         if ((rc = dalloc(h, &h->S2, h->S_bytes))) return bail(rc);
-    } else if (h->evolve_gw && !h->fftp && !(p->flags & GABE_FLAG_NO_OVERLAP)) {
+    } else if (h->evolve_gw && !(h->fftp && h->N >= 128) && !(p->flags & GABE_FLAG_NO_OVERLAP)) {
+        // (the plane form runs in line from 128^3 on: overlapped 147 against 151 us a step there, but 190 against 184
+        // with the energies read after each; below, overlapped 18.5 against 23.7 us at 16^3, 24.8 against 31.8 at 48^3,
+        // 75 against 80 at 96^3)
         // optional: without it the GW chain simply runs in line
         if (dalloc(h, &h->S2, h->S_bytes) != GABE_OK) {
             h->S2 = nullptr;

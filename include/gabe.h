@@ -72,8 +72,8 @@ enum gabe_flags {
                                  words of device memory).  With the library's 3-D FFT the chain runs
                                  in line anyway and the second buffer is the target of its column
                                  passes (out of place, faster); this flag makes them in place.  The
-                                 transposed transform needs the second buffer in any case, the plane
-                                 transform never does */
+                                 transposed transform needs the second buffer in any case; the plane
+                                 transform has one below N = 128, for the overlap only */
     GABE_FLAG_OWN_FFT = 16,     /* FP32 with N in {64, 128, 256, 512}: transform the GW sources with the
                                    library's in-layout three-pass 3-D r2c (the layout of a library r2c)
                                    followed by the separate k-space pass, instead of the default */
@@ -88,7 +88,7 @@ enum gabe_flags {
                                    pass along i fused with the TT projection and h/l update, so the
                                    transformed sources are never written back.  The default for FP32 at
                                    N in {256, 512} (the fastest form measured there on B200; the plane
-                                   transform is ahead by 4 % at 128, cuFFT's plan ties at 64); needs the
+                                   transform is ahead by 5 % at 128, cuFFT's plan ties at 64); needs the
                                    second source buffer whatever GABE_FLAG_NO_OVERLAP says */
 };
 

@@ -528,9 +528,10 @@ int gabe_create(const gabe_params *p, gabe_handle **out) {
     h->fftt = h->evolve_gw && h->f32 && fftt_supported(h->N) &&
               ((p->flags & GABE_FLAG_TRANSPOSED_FFT) ||
                (h->N >= 128 && !(p->flags & (GABE_FLAG_OWN_FFT | GABE_FLAG_CUFFT_3D))));
-    // the plane transform at the sizes it takes except 64, unless a flag names a form: a step at 96^3 80 us against
-    // 125 with cuFFT's plan and its chain overlapped, at 128^3 152 against 160 with the transposed form, at 160^3 323
-    // against 425; at 64^3, where every launch is short, 39.0 against 36.9 with cuFFT's overlapped chain
+    // the plane transform at the sizes it takes except 64, unless a flag names a form: a step at 48^3 24.8 us against
+    // 28.9 with cuFFT's plan and its overlapped chain, at 96^3 75 against 125, at 128^3 152 against 158 with the
+    // transposed form, at 160^3 323 against 425.  64^3 stays with cuFFT's plan (36.0 us; the plane form in line took
+    // 39.0, overlapped 29.9)
     h->fftp = h->evolve_gw && h->f32 && fftp_supported(h->N) && h->N != 64 &&
               !(p->flags & (GABE_FLAG_OWN_FFT | GABE_FLAG_CUFFT_3D | GABE_FLAG_TRANSPOSED_FFT));
     if (h->fftp) h->fftt = false;

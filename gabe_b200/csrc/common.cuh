@@ -5,9 +5,9 @@
 //   momenta  D[buf][fld][i][j][k]
 //   GW       h[12][i][j][kz], l[12][i][j][kz]   planar, kz < N/2+1
 //   sources  S[10][i][j][row]  real: 11,12,13,22,23 of stage 0, then of
-//            stage 1; rows of N + 2 where the transform runs in place (the
-//            same bytes then hold the half spectra S^[10][i][j][kz]), of N
-//            where it writes a second array (FP32)
+//            stage 1; rows of N + 2 (an in-place r2c then leaves the half
+//            spectra S^[10][i][j][kz] in the same bytes) or, FP32, of N
+//            (SrcLayout in stencil.cuh)
 //   scalars  DevScalars (a, adot, energies per stage, homogeneous
 //            trajectory of the FP32 path, status word)
 //   partials per-block FP64 sums of the energy reductions

@@ -11,8 +11,9 @@
 //     that finishes the last item of a lattice, in item order, so every
 //     lattice gets its own Friedmann update without a grid-wide barrier;
 //   * the GW transforms and the k-space update are the plane transform's two
-//     launches (fftp.cuh) per batch of lattices of one size, a batch's
-//     transformed planes small enough to stay in L2 between them;
+//     launches (fftp.cuh) per batch of lattices of one size, batches
+//     alternating on two side streams, so that one's lines run beside the
+//     next one's planes;
 //   * at sizes the plane transform does not take: one cuFFT call per lattice
 //     size (batch = 10 x lattices of that size, sources of a size group
 //     contiguous) and one k-space kernel over those lattices, in chunks of
@@ -34,7 +35,7 @@ namespace gabe {
 struct EnsLat {
     LatticeConsts c;
     float *X[2], *D[2];  // [2 fields][N^3] each, ping-pong
-    float *S;            // [10][N][N][N+2] sources / [..][N][N][N/2+1] spectra
+    float *S;            // ten arrays of N N (N + 2) reals: sources (SRC_PLANES or SRC_PADDED), then their transforms
     Cplx<float> *G;      // [4][M] h+, hx, l+, lx
     DevScalars *sc;
     int gt;              // order of G (g_index): 2 with the plane transform, 0 with cuFFT's
@@ -105,7 +106,7 @@ __global__ void __launch_bounds__(kEnsThreads, s32::sweep32_threads_per_sm<MODE>
     t.planes = 0;
     t.src = L.gt == 2 ? SRC_PLANES : SRC_PADDED;
     __shared__ s32::Site32 s;
-    // by a warp that copies nothing; the march waits for the block before it reads them
+    // by the last thread, which copies nothing; the march waits for the block before it reads them
     if (tid == (int)blockDim.x - 1) s32::site32_consts<MODE>(c, L.sc, s);
     double acc[kNV];
 #pragma unroll

@@ -785,8 +785,9 @@ __global__ void __launch_bounds__(NT, 1)
 // other tile's MMAs have SiLU to run under there too.
 // Results are those of the layer-by-layer kernels bit for bit: the same
 // products in the same K order, the same epilogue arithmetic.
-// Measured (1M rows, default network): 0.80 ms against 1.02 for the five
-// launches; 41 rows 27 us a call against 47.  What set the pace on the way
+// Measured at 1965 MHz: 1M rows through the default network 0.86 ms a call
+// (calls queued one behind another) against 1.02 for the five launches, 41
+// rows 27 us a call waited for against 47.  What set the pace on the way
 // there, read from clock stamps: divisions and remainders in the two issuing
 // threads (1000 cycles per weight slot beside 16 busy warps; 1.2 ms), 16 KB
 // slots (twice the waits and commits of 32 KB ones), a first layer by a lane

@@ -36,7 +36,7 @@ __device__ __forceinline__ double field_value(const OutArgs &a, int fld, size_t 
 // mean, and its sum is dominated by that mean's rounding, so each thread's
 // order of additions is part of the result).  The loads of kMvUnroll
 // iterations are issued together, the additions stay in order.
-constexpr int kMvUnroll = 8;
+constexpr int kMvUnroll = 4;
 static __global__ void __launch_bounds__(256) meansvars_kernel(OutArgs a, int pass) {
     __shared__ double sred[8 * 2];
     __shared__ int sflag;

@@ -52,7 +52,7 @@ struct StencilArgs {
     const void *D;       // momenta in [2][N^3]
     void *Xo;            // fields out   (sweep B)
     void *Do;            // momenta out  (sweep B)
-    void *S;             // GW sources [10][N][N][N+2] (sweep A with GWs)
+    void *S;             // GW sources (sweep A with GWs); FP32 in the layout src, FP64 [10][N][N][N+2]
     double *partials;    // [nblocks][8]
     unsigned int *counter;
     DevScalars *sc;

@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(TK2 *TJ, (sweep32_threads_per_sm<MODE>() + TK2
     t.i1 = min(t.i0 + args.ci, end);
 
     __shared__ Site32 s;
-    // by a warp that copies nothing; the march waits for the block before it reads them
+    // by the last thread, which copies nothing; the march waits for the block before it reads them
     if (tid == (int)blockDim.x - 1) site32_consts<MODE>(c, args.sc, s);
     double acc[kNV];
 #pragma unroll

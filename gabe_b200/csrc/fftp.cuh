@@ -27,10 +27,12 @@
 // separated without their factor 1/2, which kspace_apply's source
 // coefficients take in, an exact power of two).
 //
-// The plane pass is bound by the load/store unit's data path (ncu at 128^3: 53 % of its wavefronts
-// over the whole launch, issue 28 %, HBM 14 %: the sources come from the L2), so the work layout is chosen for conflict-free accesses (place)
-// and the pass writes its planes as they lie; the lines pass by the latency
-// of its loads behind three barriers (two CTAs of 82 KB per SM at 128^3).
+// The plane pass is bound by the load/store unit's data path (ncu at 128^3:
+// 53 % of its wavefronts over the whole launch, issue 28 %, HBM 14 %: the
+// sources come from the L2), so the work layout is chosen for conflict-free
+// accesses (place) and the pass writes its planes as they lie; the lines pass
+// by the latency of its loads behind three barriers (two CTAs of 82 KB per SM
+// at 128^3).
 // Measured on B200, GW transforms + k-space update of one step: 96^3 53 us
 // against 107 for cuFFT's plan and the separate pass, 128^3 110 against 148
 // (116 for the three passes of fftt.cuh), 160^3 240 against 339; the

@@ -144,19 +144,20 @@ __device__ __forceinline__ ModelP model_p(const LatticeConsts &c) {
     return ModelP{k(-c.mc[0]), k(-c.mc[1]), k(c.mc[1]), k(c.mc[2]), k(c.mc[3]), f2(0.5f)};
 }
 
-// Takes V'(fbar+d) - V'(fbar) of both fields off t.
+// Takes V'(fbar+d) - V'(fbar) of both fields off t (SET: off zero).
+template <bool SET>
 __device__ __forceinline__ void sub_dv_diff32(const MeanP &m, const ModelP &q, int model, F2 a, F2 b, F2 (&t)[2]) {
     const F2 C = m.cb + b;
     const F2 u = fma2(a, C * C, (m.pb * b) * (m.cb2 + b));  // pb b (2 cb + b) + a C^2
     const F2 w = fma2(a * (m.pb2 + a), C, m.pbsq * b);
     if (model == MODEL_QUADRATIC) {
         // V' = phi + C1 chi^2 phi ; V'_chi = C1 phi^2 chi
-        t[0] = fma2(q.n0, u, t[0] - a);
-        t[1] = fma2(q.n0, w, t[1]);
+        t[0] = (SET ? q.n0 * u : fma2(q.n0, u, t[0])) - a;
+        t[1] = SET ? q.n0 * w : fma2(q.n0, w, t[1]);
     } else {
         // V' = lam phi^3 + g chi^2 phi ; V'_chi = g phi^2 chi
-        t[0] = fma2(q.n0 * a, fma2(a, m.pbt + a, m.pb3sq), fma2(q.n1, u, t[0]));
-        t[1] = fma2(q.n1, w, t[1]);
+        t[0] = fma2(q.n0 * a, fma2(a, m.pbt + a, m.pb3sq), SET ? q.n1 * u : fma2(q.n1, u, t[0]));
+        t[1] = SET ? q.n1 * w : fma2(q.n1, w, t[1]);
     }
 }
 

@@ -124,14 +124,20 @@ __device__ __forceinline__ Pair pair_of(F2 m6, F2 cu, F2 nx, F2 pr, F2 up, F2 dn
     return p;
 }
 
+// In the force, lap / a^2 - V' - 3 H d, the Laplacian is the largest term by far, but the mean of V' over the lattice is
+// what drives the mean field.  So V' and the drag are summed first and the Laplacian's product enters last and
+// unrounded: one rounding at its size, and one that is as often up as down.  Added to a rounded Laplacian, the part of V'
+// below half an ulp of it was lost, always in the same direction (potential energy off by 1.7e-13 instead of 1e-15 after
+// 150 steps at 128^3, lambda phi^4; by 3.9e-11 instead of 1e-14 after 1000 at 512^3).
+
 // The thread's pair of sites in sweep A / E0: adds to the moments, fills the sources.
 template <int MODE, int MODEL = -1>
 __device__ __forceinline__ void site_a32(const LatticeConsts &c, const Site32 &s, const Pair (&p)[4], Moments &m,
                                          F2 (&s0)[kSrc], F2 (&s1)[kSrc]) {
     const int model = site_model<MODEL>(c);
     const F2 h = s.h;
-    F2 t0[2] = {s.k0 * p[0].lap, s.k0 * p[1].lap}, f1[2];  // stage-0 force without the drag
-    if constexpr (MODE != MODE_E0) sub_dv_diff32(s.m0, s.q, model, p[0].v, p[1].v, t0);
+    F2 t0[2], f1[2];
+    if constexpr (MODE != MODE_E0) sub_dv_diff32<true>(s.m0, s.q, model, p[0].v, p[1].v, t0);
     F2 P0[6], P1[6];
     if constexpr (MODE == MODE_A_GW) {
 #pragma unroll
@@ -146,7 +152,7 @@ __device__ __forceinline__ void site_a32(const LatticeConsts &c, const Site32 &s
         m.g0 = fma2(ff.v, ff.lap, m.g0);
         if constexpr (MODE != MODE_E0) {
             f1[f] = fma2(h, d, ff.v);
-            const F2 Pd = fma2(h, t0[f], d);
+            const F2 Pd = fma2(h, fma2(s.k0, ff.lap, t0[f]), d);  // stage-0 force without the drag
             m.c[f] = m.c[f] + Pd;
             m.e = fma2(Pd, Pd, m.e);
             m.f = fma2(Pd, d, m.f);
@@ -174,19 +180,20 @@ __device__ __forceinline__ void site_b32(const LatticeConsts &c, const Site32 &s
     F2 t0[2], t1[2], f1[2], d1[2];
 #pragma unroll
     for (int f = 0; f < 2; f++) {
-        t0[f] = fma2(s.n3H0, p[2 + f].v, s.k0 * p[f].lap);
+        t0[f] = s.n3H0 * p[2 + f].v;
         f1[f] = fma2(h, p[2 + f].v, p[f].v);
     }
-    sub_dv_diff32(s.m0, s.q, model, p[0].v, p[1].v, t0);
+    sub_dv_diff32<false>(s.m0, s.q, model, p[0].v, p[1].v, t0);
 #pragma unroll
     for (int f = 0; f < 2; f++) {
-        d1[f] = fma2(h, t0[f], p[2 + f].v);
+        d1[f] = fma2(h, fma2(s.k0, p[f].lap, t0[f]), p[2 + f].v);
         xo[f] = fma2(dt, d1[f], p[f].v);
-        t1[f] = fma2(s.n3H1, d1[f], s.k1 * fma2(h, p[2 + f].lap, p[f].lap));
+        t1[f] = s.n3H1 * d1[f];
     }
-    sub_dv_diff32(s.m1, s.q, model, f1[0], f1[1], t1);
+    sub_dv_diff32<false>(s.m1, s.q, model, f1[0], f1[1], t1);
 #pragma unroll
-    for (int f = 0; f < 2; f++) dout[f] = fma2(dt, t1[f], p[2 + f].v);
+    for (int f = 0; f < 2; f++)
+        dout[f] = fma2(dt, fma2(s.k1, fma2(h, p[2 + f].lap, p[f].lap), t1[f]), p[2 + f].v);
 }
 
 // Threads per SM the register budget is sized for: sweep A with sources holds

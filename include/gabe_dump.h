@@ -118,15 +118,16 @@ static inline int gabe_dump_read(const char *path, gabe_dump_header *hd, double 
  * field and momenta of stage 0 (field_bytes each: FP64 values, or for
  * FP32 storage the FP32 fluctuations about the homogeneous trajectory kept
  * in the scalar block) and, with GWs, the four TT amplitudes h+, hx, l+,
- * lx (gw_bytes; complex, [4][i][j][kz] for gw_layout 0 or [4][kz][j][i]
- * for gw_layout 1).  Loading the block into a handle of the same precision,
- * amplitude layout and tile plan continues the run bit for bit. */
+ * lx (gw_bytes; complex, [4][i][j][kz] for gw_layout 0, [4][kz][j][i] for 1,
+ * [4][x / 8][i][x % 8] with x = j (N/2+1) + kz for 2).  Loading the block
+ * into a handle of the same precision, transform form and tile plan continues
+ * the run bit for bit; FP32 amplitudes of another layout are reordered. */
 #define GABE_RESTART_MAGIC "GABERST1"
 
 typedef struct {
     char magic[8];
     int32_t precision;      /* enum gabe_precision of the writer */
-    int32_t gw_layout;      /* 0 [4][i][j][kz], 1 [4][kz][j][i] */
+    int32_t gw_layout;      /* order of the amplitudes, 0 to 2 as above */
     int32_t expansion;
     int32_t tile_shape, tile_ci;
     int32_t e0_stale;       /* the stage-0 energies of the scalar block were not yet reduced */

@@ -20,7 +20,7 @@
 // The sweeps were bound by instruction issue, not by HBM: with one site per
 // instruction, the neighbours' stage-1 values formed one by one, separate own
 // and halo copies and the constants in registers a warp took 424 instructions
-// per plane of sweep A (370 sweep B), now 210 (188).  At 256^3, fields only:
+// per plane of sweep A (370 sweep B), now 211 (191).  At 256^3, fields only:
 // sweep A 118 against 152 us, B 111 against 119 (its 537 MB take 82 at the
 // measured copy rate), energies alone 107 against 118.  With GW sources the
 // stores bound sweep A.

@@ -1685,7 +1685,10 @@ int launch_fused(gabe_mlp *m, const float *x, int rows, float *y, bool keep) {
 // With BF16 activations every layer after the first runs on tensor cores.
 template <typename TACT>
 int forward_rows(gabe_mlp *m, const float *x, int rows, float *y, bool keep_z) {
-    if (m->fused_slots) {
+    // The one-launch form stores a tile's outputs while other tiles' inputs are still to be read: an output that
+    // overlaps the inputs takes the layers, the first of which reads them all.
+    const float *xe = x + (long long)rows * m->p.n_in, *ye = y + (long long)rows * m->p.n_out;
+    if (m->fused_slots && (xe <= y || ye <= x)) {
         const int rc = launch_fused(m, x, rows, y, keep_z);
         if (rc != kNoTensorMap) return rc;  // else: e.g. an output pointer off a 16-byte boundary
     }

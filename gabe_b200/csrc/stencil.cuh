@@ -490,7 +490,9 @@ __device__ __forceinline__ void finish_b(const LatticeConsts &c, DevScalars *s) 
 // what the march does for the other states, without its speed (sweep A's sources, which hold no quotient, are not
 // written again).  Out of line, on no local of the march and with little in registers, so that the march keeps its
 // own: a second march inlined beside the first cost sweep A at 256^3 without GW sources 276 us against 252, this
-// nothing (with sources 487 us against 512: 128 registers instead of 154).
+// nothing (with sources 507-517 us against 538-542).  A step without it takes 2 % less where the columns are 8 x 8
+// (200^3 with GWs 2.08 ms against 2.13) or a block's march is short (100^3 112 us against 114), 1-2 % more at 180^3
+// and 252^3, and the same within 1 % at 64^3, 128^3, 240^3 and 256^3: the march is scheduled another way.
 template <int MODE>
 __device__ __noinline__ void sites_inf(const StencilArgs &args, int i0, int i1, int j, int k, double *sums) {
     const LatticeConsts &c = args.c;

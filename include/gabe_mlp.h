@@ -63,7 +63,8 @@ int64_t gabe_mlp_num_params(const gabe_mlp *m);
 int gabe_mlp_set_params(gabe_mlp *m, const float *h_params);
 int gabe_mlp_get_params(gabe_mlp *m, float *h_params);
 
-/* y [n][n_out] = net(x [n][n_in]); any n >= 0 (processed in chunks of max_rows). */
+/* y [n][n_out] = net(x [n][n_in]); any n >= 0 (processed in chunks of max_rows).
+ * y may overlap x where n <= max_rows (the layers then run one by one). */
 int gabe_mlp_forward(gabe_mlp *m, const float *x, int64_t n, float *y);
 
 /* Loss and gradient of one batch (n <= max_rows), for checks: h_loss = mean
